@@ -305,23 +305,24 @@ void* wake_grid_state_buffer(wake_grid* g, int which);
 /* Launch shape of the fused kernel: threads per block (32..512, multiple of 32). */
 int wake_grid_set_block(wake_grid* g, int threads_per_block);
 int wake_grid_get_block(wake_grid* g);
-/* Step kernels: 0 automatic (default), 1 direct (a launch over the pure-gather
- * spans reading global memory, beside a launch over the remaining rows), 2 one
- * persistent launch per step that stages the pure-gather rows in shared memory
- * by bulk copies, tiles of up to 1024 nodes, and runs the remaining rows beside
- * them (used when a row is a whole number of 16-byte chunks and at most 1024
- * nodes), 3 (TRT) one block per row whose every node is a pure gather, 4 (TRT)
- * those rows moved through shared memory by bulk copies in both directions, a
- * few rows in flight per block (rows of at most 512 nodes and a whole number of
- * 16-byte chunks). A variant whose conditions do not hold runs the direct
- * kernels. Automatic: 4 for 16-bit storage where it applies, else 1.
- * get_kernel prepares the grid and returns the variant in use (1 to 4). For
- * TRT every variant computes two nodes per thread in packed FP32 with the same
- * roundings, so all give the same bits. No reference counterpart. */
+/* Step kernels: 0 automatic (default), 1 direct (one launch of the whole
+ * lattice reading global memory), 2 one persistent launch per step that stages
+ * the rows of pure gathers in shared memory by bulk copies, tiles of up to 1024
+ * nodes, beside the direct kernel on the remaining rows (used when a row is a
+ * whole number of 16-byte chunks and at most 1024 nodes, without a coupled
+ * temperature), 3 (TRT) one block per row whose every node is a pure gather, 4
+ * (TRT) those rows moved through shared memory by bulk copies in both
+ * directions, a few rows in flight per block (rows of at most 512 nodes and a
+ * whole number of 16-byte chunks). A variant whose conditions do not hold runs
+ * the direct kernel. Automatic: 4 for 16-bit storage where it applies, else 1.
+ * get_kernel prepares the grid and returns the variant in use (1 to 4). Every
+ * variant computes a node in the same way, so all give the same bits. No
+ * reference counterpart. */
 int wake_grid_set_kernel(wake_grid* g, int variant);
 int wake_grid_get_kernel(wake_grid* g);
-/* Kernel launches one fused step issues with the current geometry (pure-gather
- * rows, general rows, momentum-exchange reduction). No reference counterpart. */
+/* Kernel launches one step issues with the current geometry: one, or with a
+ * row variant (2 to 4) one for its rows and one for the others. No reference
+ * counterpart. */
 int wake_grid_launches_per_step(wake_grid* g);
 /* CUDA-event timing of each pure-gather (bulk) launch. While on, steps run as
  * plain launches (no graph). bulk_launch_times synchronizes, returns the summed
@@ -386,9 +387,10 @@ int wake_batch_remove(wake_batch* b, wake_grid* g);
 int wake_batch_size(wake_batch* b);
 int wake_batch_set_stream(wake_batch* b, void* stream);
 int wake_batch_use_graph(wake_batch* b, int steps_per_graph);
+/* threads_bulk: threads per block of the one launch of a step (threads_general is accepted and unused). */
 int wake_batch_set_block(wake_batch* b, int threads_bulk, int threads_general);
 int wake_batch_get_block(wake_batch* b);
-/* As wake_grid_set_kernel, for the batch (persistent tiles only when every member allows them). */
+/* Accepts 0, 1 and 2; a batch steps with the direct kernel, whose results every variant shares. */
 int wake_batch_set_kernel(wake_batch* b, int variant);
 int wake_batch_step(wake_batch* b, int n);
 int wake_batch_synchronize(wake_batch* b);        /* first member error, if any */

@@ -3,11 +3,8 @@
 // LatticeGrid per object and call (src/grid/lattice_grid_2d.cpp:195-265); a
 // parameter sweep or a serving loop runs one such object per job. Here every
 // member keeps its own state, geometry, parameters and force history (it is an
-// ordinary wake_grid), and one step of the whole batch is three launches:
-//
-//   bulk launch    : every pure-gather row of every member (k_step_fast_batch)
-//   general launch : every other row (k_step_batch), on a forked stream
-//   reduction      : one block per member with momentum exchange
+// ordinary wake_grid), and one step of the whole batch is one launch of k_step_cells_batch: the listed cells of
+// every member, then the pure cells of every member.
 //
 // Each launch reads the member's step arguments from a device table, so members
 // of any size share a launch and the per-node arithmetic is the single-lattice
@@ -19,23 +16,6 @@
 
 #include "engine.cuh"
 
-namespace wk {
-
-struct MemRed {  // one member's momentum-exchange reduction
-    const double* contrib;
-    int n;
-    unsigned* hist_step;
-    double* hist;
-    int hist_cap;
-};
-
-__global__ void __launch_bounds__(256) k_batch_mem_reduce(const MemRed* __restrict__ list) {
-    const MemRed m = list[blockIdx.x];
-    mem_reduce_block(m.contrib, m.n, m.hist_step, m.hist, m.hist_cap);
-}
-
-}  // namespace wk
-
 using namespace wk;
 
 struct wake_batch {
@@ -45,51 +25,38 @@ struct wake_batch {
     };
     int Q = 0, storage = 0;
     std::vector<Member> members;
-    cudaStream_t stream = nullptr, side = nullptr;
+    cudaStream_t stream = nullptr;
     bool own_stream = false;
-    cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
 
-    DevMem d_dom, d_fast, d_gen, d_red;
+    DevMem d_dom, d_pure, d_listed;
     std::vector<BatchDom> up_dom;  // table as last uploaded
-    std::vector<MemRed> up_red;
-    int n_fast = 0, n_gen = 0, n_red = 0;
-    bool idx32 = true;
-    bool tiles = false;      // one persistent tile launch per step (k_step_tiles)
-    int kernel_variant = 0;  // 0 automatic, 1 direct, 2 persistent tiles (when every member allows it)
-    DevMem d_tiles, d_gen4, d_mixed;  // tiles, general segments with entries, spans outside the tiles
-    int n_tiles = 0, n_tile_gen = 0, n_mixed = 0;
+    int n_pure = 0, n_listed = 0;
+    bool thermal = false;  // some member has a coupled temperature
+    long long state_bytes = 0;  // one state buffer of every member
     int coll = 0, les = 0;
     int parity = 0;  // batch steps taken, mod 2
 
     // row lists are rebuilt when the members or any member's geometry change
     std::vector<std::pair<const wake_grid*, unsigned long long>> layout;
-    std::vector<int> gen_first;
     unsigned shape = 0;  // bumped when launch shapes or table addresses change
     // host seconds spent in wake_batch_step: preparing members and tables, capturing and
     // instantiating graphs, issuing launches (a launch that waits for queue space counts here)
     double host_s[3] = {0.0, 0.0, 0.0};
 
-    int tpb_fast = 64, tpb_gen = 128;
+    int tpb = 64;
 
     cudaGraphExec_t graph = nullptr;
     int graph_steps = 0, graph_parity = -1;
     unsigned graph_shape = ~0u;
 
     ~wake_batch() {
-        if (stream && cudaStreamSynchronize(stream) == cudaSuccess && (!side || cudaStreamSynchronize(side) == cudaSuccess)) {
+        if (stream && cudaStreamSynchronize(stream) == cudaSuccess) {
             d_dom.release();
-            d_fast.release();
-            d_gen.release();
-            d_red.release();
-            d_tiles.release();
-            d_gen4.release();
-            d_mixed.release();
+            d_pure.release();
+            d_listed.release();
         }
         if (graph) cudaGraphExecDestroy(graph);
         if (own_stream && stream) cudaStreamDestroy(stream);
-        if (side) cudaStreamDestroy(side);
-        if (ev_fork) cudaEventDestroy(ev_fork);
-        if (ev_join) cudaEventDestroy(ev_join);
     }
     void drop_graph() {
         if (graph) cudaGraphExecDestroy(graph);
@@ -108,68 +75,63 @@ bool valid_batch(wake_batch* b) {
     return true;
 }
 
-// Rebuild the concatenated row lists when the membership or a member's geometry changed.
-int build_rows(wake_batch* b) {
+// Rebuild the concatenated cell lists when the membership or a member's geometry changed.
+int build_cells(wake_batch* b) {
     std::vector<std::pair<const wake_grid*, unsigned long long>> layout;
     layout.reserve(b->members.size());
-    for (const auto& m : b->members) layout.emplace_back(m.g, m.g->geom_version);
-    if (layout == b->layout && b->gen_first.size() == b->members.size()) return WAKE_OK;
+    for (const auto& m : b->members) layout.emplace_back(m.g, m.g->units_version);
+    if (layout == b->layout) return WAKE_OK;
     // queued steps may still read the old lists: let them finish, then lists can move freely
     WK_CUDA(cudaStreamSynchronize(b->stream));
-    if (b->side) WK_CUDA(cudaStreamSynchronize(b->side));
-    std::vector<uint4> fast, tiles, gen4, mixed;
-    std::vector<uint2> gen;
-    b->gen_first.assign(b->members.size(), 0);
+    std::vector<uint2> pure, listed;
     for (std::size_t i = 0; i < b->members.size(); ++i) {
         const wake_grid* g = b->members[i].g;
         const unsigned m = static_cast<unsigned>(i);
-        for (uint4 sp : g->h_fast_rows) fast.push_back(make_uint4(m, sp.y, sp.z, sp.w));
-        b->gen_first[i] = static_cast<int>(gen.size());
-        for (unsigned r : g->h_gen_rows) gen.push_back(make_uint2(m, r));
-        for (uint4 t : g->h_tiles) tiles.push_back(make_uint4(m, t.y, t.z, 0u));
-        for (uint4 t : g->h_gen4) gen4.push_back(make_uint4(m, t.y, t.z, 0u));
-        for (uint4 sp : g->h_mixed) mixed.push_back(make_uint4(m, sp.y, sp.z, sp.w));
+        if (!g->narrow()) continue;  // stepped by its own launches
+        if (g->mem_on) listed.push_back(make_uint2(m, LISTED_SUM));
+        for (unsigned w : g->cells.units)
+            if (!(w & UNIT_PURE)) listed.push_back(make_uint2(m, w));
+        // its pure cells, linear and listed, in node order
+        const auto cell = [&](unsigned i, unsigned nodes, bool zh) {
+            pure.push_back(make_uint2(m | (nodes - 1u) << 24 | (zh ? 1u << 30 : 0u), i));
+        };
+        unsigned e = g->cells.general;
+        const std::vector<uint4>& list = g->cells.cells;
+        const auto listed_before = [&](unsigned i) {
+            for (; e < list.size() && list[e].x < i; ++e) cell(list[e].x, list[e].y & 0xffu, list[e].y & LIST_ZH);
+        };
+        for (std::size_t c = 0; c < g->h_kind.size(); ++c) {
+            if (!(g->h_kind[c] & CELL_PURE)) continue;
+            const unsigned i = static_cast<unsigned>(c) * CELL;
+            listed_before(i);
+            cell(i, std::min<unsigned>(CELL, static_cast<unsigned>(g->N) - i), g->h_kind[c] & CELL_ZH);
+        }
+        listed_before(0xffffffffu);
     }
-    WK_CUDA(b->d_mixed.grow(sizeof(uint4) * std::max<std::size_t>(1, mixed.size())));
-    if (!mixed.empty())
-        WK_CUDA(cudaMemcpyAsync(b->d_mixed.p, mixed.data(), sizeof(uint4) * mixed.size(), cudaMemcpyHostToDevice,
+    WK_CUDA(b->d_pure.grow(sizeof(uint2) * std::max<std::size_t>(1, pure.size())));
+    WK_CUDA(b->d_listed.grow(sizeof(uint2) * std::max<std::size_t>(1, listed.size())));
+    if (!pure.empty())
+        WK_CUDA(cudaMemcpyAsync(b->d_pure.p, pure.data(), sizeof(uint2) * pure.size(), cudaMemcpyHostToDevice, b->stream));
+    if (!listed.empty())
+        WK_CUDA(cudaMemcpyAsync(b->d_listed.p, listed.data(), sizeof(uint2) * listed.size(), cudaMemcpyHostToDevice,
                                 b->stream));
-    b->n_mixed = static_cast<int>(mixed.size());
-    WK_CUDA(b->d_tiles.grow(sizeof(uint4) * std::max<std::size_t>(1, tiles.size())));
-    WK_CUDA(b->d_gen4.grow(sizeof(uint4) * std::max<std::size_t>(1, gen4.size())));
-    if (!tiles.empty())
-        WK_CUDA(cudaMemcpyAsync(b->d_tiles.p, tiles.data(), sizeof(uint4) * tiles.size(), cudaMemcpyHostToDevice,
-                                b->stream));
-    if (!gen4.empty())
-        WK_CUDA(cudaMemcpyAsync(b->d_gen4.p, gen4.data(), sizeof(uint4) * gen4.size(), cudaMemcpyHostToDevice,
-                                b->stream));
-    b->n_tiles = static_cast<int>(tiles.size());
-    b->n_tile_gen = static_cast<int>(gen4.size());
-    WK_CUDA(b->d_fast.grow(sizeof(uint4) * std::max<std::size_t>(1, fast.size())));
-    WK_CUDA(b->d_gen.grow(sizeof(uint2) * std::max<std::size_t>(1, gen.size())));
-    if (!fast.empty())
-        WK_CUDA(cudaMemcpyAsync(b->d_fast.p, fast.data(), sizeof(uint4) * fast.size(), cudaMemcpyHostToDevice, b->stream));
-    if (!gen.empty())
-        WK_CUDA(cudaMemcpyAsync(b->d_gen.p, gen.data(), sizeof(uint2) * gen.size(), cudaMemcpyHostToDevice, b->stream));
     WK_CUDA(cudaStreamSynchronize(b->stream));  // the host vectors go out of scope
-    b->n_fast = static_cast<int>(fast.size());
-    b->n_gen = static_cast<int>(gen.size());
+    b->n_pure = static_cast<int>(pure.size());
+    b->n_listed = static_cast<int>(listed.size());
     b->layout = std::move(layout);
     b->up_dom.clear();  // force a table upload
     ++b->shape;
     return WAKE_OK;
 }
 
-// Step-argument table and reduction list of the current members; uploaded when changed.
+// Step-argument table of the current members; uploaded when changed.
 int build_tables(wake_batch* b) {
     const std::size_t n = b->members.size();
     std::vector<BatchDom> dom(n);
-    std::vector<MemRed> red;
-    b->idx32 = true;
-    bool tiles = b->kernel_variant == 2 && n > 0;
+    bool thermal = false;
+    b->state_bytes = 0;
     for (std::size_t i = 0; i < n; ++i) {
         wake_grid* g = b->members[i].g;
-        tiles = tiles && tile_row_ok(g->nx, static_cast<int>(g->elem));
         BatchDom d;
         std::memset(&d, 0, sizeof d);
         d.a = grid_step_args(g);
@@ -178,81 +140,46 @@ int build_tables(wake_batch* b) {
         d.tbuf[0] = g->tbuf(0);
         d.tbuf[1] = g->tbuf(1);
         d.cur0 = g->cur ^ b->parity;
-        d.gen_first = b->gen_first[i];
+        d.alone = g->narrow() ? 0 : 1;
         dom[i] = d;
-        if (static_cast<long long>(g->Q) * g->pitch >= (1ll << 32)) b->idx32 = false;
-        if (g->mem_on) {
-            MemRed m;
-            std::memset(&m, 0, sizeof m);
-            m.contrib = d.a.mem.contrib;
-            m.n = d.a.mem.n_nodes;
-            m.hist_step = d.a.mem.hist_step;
-            m.hist = d.a.mem.hist;
-            m.hist_cap = d.a.mem.hist_cap;
-            red.push_back(m);
-        }
+        thermal = thermal || g->th.on;
+        b->state_bytes += static_cast<long long>(g->elem) * g->Q * g->pitch;
     }
-    if (tiles != b->tiles) {
-        b->tiles = tiles;
+    if (thermal != b->thermal) {
+        b->thermal = thermal;
         ++b->shape;  // a captured graph holds the other kernel
     }
-    const bool same_dom = dom.size() == b->up_dom.size() &&
-                          (dom.empty() || std::memcmp(dom.data(), b->up_dom.data(), sizeof(BatchDom) * n) == 0);
-    const bool same_red = red.size() == b->up_red.size() &&
-                          (red.empty() || std::memcmp(red.data(), b->up_red.data(), sizeof(MemRed) * red.size()) == 0);
-    if (same_dom && same_red) return WAKE_OK;
-    WK_CUDA(cudaStreamSynchronize(b->stream));  // queued steps may still read the old tables
-    if (b->side) WK_CUDA(cudaStreamSynchronize(b->side));
+    if (dom.size() == b->up_dom.size() &&
+        (dom.empty() || std::memcmp(dom.data(), b->up_dom.data(), sizeof(BatchDom) * n) == 0))
+        return WAKE_OK;
+    WK_CUDA(cudaStreamSynchronize(b->stream));  // queued steps may still read the old table
     const void* old_dom = b->d_dom.p;
-    const void* old_red = b->d_red.p;
-    const int old_nred = b->n_red;
     WK_CUDA(b->d_dom.grow(sizeof(BatchDom) * std::max<std::size_t>(1, n)));
-    WK_CUDA(b->d_red.grow(sizeof(MemRed) * std::max<std::size_t>(1, red.size())));
     if (n) WK_CUDA(cudaMemcpyAsync(b->d_dom.p, dom.data(), sizeof(BatchDom) * n, cudaMemcpyHostToDevice, b->stream));
-    if (!red.empty())
-        WK_CUDA(cudaMemcpyAsync(b->d_red.p, red.data(), sizeof(MemRed) * red.size(), cudaMemcpyHostToDevice, b->stream));
     WK_CUDA(cudaStreamSynchronize(b->stream));
-    b->n_red = static_cast<int>(red.size());
     b->up_dom = std::move(dom);
-    b->up_red = std::move(red);
     // a captured graph keeps launch shapes and table addresses, not the table contents
-    if (old_dom != b->d_dom.p || old_red != b->d_red.p || old_nred != b->n_red) ++b->shape;
+    if (old_dom != b->d_dom.p) ++b->shape;
     return WAKE_OK;
 }
 
 int batch_steps(wake_batch* b, int n) {
-    if (b->tiles) {
-        for (int s = 0; s < n; ++s) {
-            const TileArgs t{b->d_tiles.as<uint4>(), b->n_tiles, b->d_gen4.as<uint4>(), b->n_tile_gen,
-                             b->d_dom.as<BatchDom>(), b->parity, b->d_mixed.as<uint4>(), b->n_mixed};
-            StepArgs unused{};
-            WK_CUDA(launch_tiles_any(b->Q, b->coll, b->storage, b->les != 0, unused, t, b->stream));
-            if (b->n_red > 0) {
-                k_batch_mem_reduce<<<b->n_red, 256, 0, b->stream>>>(b->d_red.as<MemRed>());
-                WK_CUDA(cudaGetLastError());
-            }
-            b->parity ^= 1;
-        }
-        return WAKE_OK;
-    }
     for (int s = 0; s < n; ++s) {
-        BatchArgs fa{b->d_dom.as<BatchDom>(), nullptr, 0, b->parity, b->d_fast.as<uint4>(), b->n_fast};
-        BatchArgs ga{b->d_dom.as<BatchDom>(), b->d_gen.as<uint2>(), b->n_gen, b->parity, nullptr, 0};
-        const bool fork = b->n_fast > 0 && (b->n_gen > 0 || b->n_red > 0);
-        cudaStream_t side = fork ? b->side : b->stream;
-        if (fork) {
-            WK_CUDA(cudaEventRecord(b->ev_fork, b->stream));
-            WK_CUDA(cudaStreamWaitEvent(b->side, b->ev_fork, 0));
-        }
-        WK_CUDA(launch_batch_any(b->Q, b->coll, b->storage, b->les != 0, ga, b->tpb_gen, side, false, b->idx32));
-        if (b->n_red > 0) {
-            k_batch_mem_reduce<<<b->n_red, 256, 0, side>>>(b->d_red.as<MemRed>());
-            WK_CUDA(cudaGetLastError());
-        }
-        WK_CUDA(launch_batch_any(b->Q, b->coll, b->storage, b->les != 0, fa, b->tpb_fast, b->stream, true, b->idx32));
-        if (fork) {
-            WK_CUDA(cudaEventRecord(b->ev_join, b->side));
-            WK_CUDA(cudaStreamWaitEvent(b->stream, b->ev_join, 0));
+        BatchArgs a{};
+        a.dom = b->d_dom.as<BatchDom>();
+        a.listed = b->d_listed.as<uint2>();
+        a.nlisted = static_cast<unsigned>(b->n_listed);
+        a.pure = b->d_pure.as<uint2>();
+        a.npure = static_cast<unsigned>(b->n_pure);
+        a.parity = b->parity;
+        a.evict_first = fits_l2(b->state_bytes);
+        WK_CUDA(launch_batch_any(b->Q, b->coll, b->storage, b->les != 0, a, b->thermal, b->tpb, b->stream));
+        for (std::size_t i = 0; i < b->up_dom.size(); ++i) {
+            if (!b->up_dom[i].alone) continue;
+            wake_grid* g = b->members[i].g;
+            StepArgs one = b->up_dom[i].a;
+            grid_step_buffers(g, b->up_dom[i].cur0 ^ b->parity, one);
+            WK_CUDA(launch_cells_any(b->Q, b->coll, b->storage, b->les != 0, one, b->tpb, b->stream));
         }
         b->parity ^= 1;
     }
@@ -273,7 +200,7 @@ int batch_prepare(wake_batch* b) {
         const int r = grid_prepare(m.g);
         if (r) return r;
     }
-    int r = build_rows(b);
+    int r = build_cells(b);
     if (r) return r;
     return build_tables(b);
 }
@@ -292,9 +219,6 @@ wake_batch* wake_batch_create(int q, int storage) {
     b->storage = storage;
     cudaError_t e = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) b->own_stream = true;
-    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->side, cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->ev_fork, cudaEventDisableTiming);
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->ev_join, cudaEventDisableTiming);
     if (e != cudaSuccess) {
         set_error(WAKE_ERR_CUDA, std::string("wake_batch_create: ") + cudaGetErrorString(e));
         delete b;
@@ -377,21 +301,17 @@ int wake_batch_set_block(wake_batch* b, int threads_bulk, int threads_general) {
         threads_general > 512 || threads_general % 32)
         return set_error(WAKE_ERR_INVALID, "wake_batch_set_block: bulk 32..256 (at most the fast kernels' bound), "
                                            "general 32..512, multiples of 32");
-    b->tpb_fast = threads_bulk;
-    b->tpb_gen = threads_general;
+    b->tpb = threads_bulk;  // one launch steps the general rows too
     b->drop_graph();
     return WAKE_OK;
 }
 
-int wake_batch_get_block(wake_batch* b) { return valid_batch(b) ? b->tpb_fast : WAKE_ERR_INVALID; }
+int wake_batch_get_block(wake_batch* b) { return valid_batch(b) ? b->tpb : WAKE_ERR_INVALID; }
 
 int wake_batch_set_kernel(wake_batch* b, int variant) {
     if (!valid_batch(b)) return WAKE_ERR_INVALID;
     if (variant < 0 || variant > 2) return set_error(WAKE_ERR_INVALID, "wake_batch_set_kernel: variant 0, 1 or 2");
-    b->kernel_variant = variant;
-    b->up_dom.clear();  // re-evaluated with the tables
-    b->drop_graph();
-    return WAKE_OK;
+    return WAKE_OK;  // every variant gives the same results; a batch has the direct kernel only
 }
 
 int wake_batch_step(wake_batch* b, int n) {
@@ -472,10 +392,10 @@ int wake_batch_info(wake_batch* b, long long* nodes, int* bulk_rows, int* genera
     long long nn = 0;
     for (const auto& m : b->members) nn += m.g->N;
     if (nodes) *nodes = nn;
-    if (bulk_rows) *bulk_rows = b->n_fast;
-    if (general_rows) *general_rows = b->n_gen;
+    if (bulk_rows) *bulk_rows = b->n_pure;
+    if (general_rows) *general_rows = b->n_listed;
     if (launches_per_step)
-        *launches_per_step = b->tiles ? 1 + (b->n_red > 0) : (b->n_fast > 0) + (b->n_gen > 0) + (b->n_red > 0);
+        *launches_per_step = b->n_pure + b->n_listed > 0 ? 1 : 0;
     return WAKE_OK;
 }
 
@@ -495,12 +415,12 @@ int wake_batch_autotune(wake_batch* b, int steps, int* best_threads) {
         cudaEventDestroy(e0);
         return set_error(WAKE_ERR_CUDA, "wake_batch_autotune: event creation failed");
     }
-    const int keep = b->tpb_fast;
+    const int keep = b->tpb;
     int best = keep;
     float best_ms = -1.f;
     for (int t : {32, 64, 128, 256}) {
         if (t > WK_FAST_MAX_THREADS) break;
-        b->tpb_fast = t;
+        b->tpb = t;
         cudaEventRecord(e0, b->stream);
         r = batch_steps(b, steps);
         cudaEventRecord(e1, b->stream);
@@ -518,9 +438,9 @@ int wake_batch_autotune(wake_batch* b, int steps, int* best_threads) {
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
-    b->tpb_fast = r ? keep : best;
+    b->tpb = r ? keep : best;
     b->drop_graph();
-    if (best_threads) *best_threads = b->tpb_fast;
+    if (best_threads) *best_threads = b->tpb;
     return r;
 }
 

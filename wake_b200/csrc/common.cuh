@@ -6,27 +6,22 @@
 #include <cstddef>
 #include <string>
 
-// Register budget of the pure-gather step kernels (k_step_fast, k_step_fast_batch): blocks of
-// at most WK_FAST_MAX_THREADS threads, at least WK_FAST_TRT_MIN_BLOCKS (TRT, two nodes per
-// thread) or WK_FAST_OTHER_MIN_BLOCKS (BGK / MRT, one node per thread) of them resident per SM.
-// 64 x 10 gives the packed TRT form 96 registers (20 warps per SM), measured 5-7% faster on the
-// D3Q19 sphere channel than 128 registers (16 warps) and 20% faster than 80 (24 warps, spills).
-// 64 x 8 lets the D3Q27 MRT step keep its moments in 106 registers without spills: 10% (FP32)
-// and 16% (FP16 / BF16) faster on the 384^3 Taylor-Green vortex than the 64-register cap.
+// Register budget of the step kernels: blocks of at most WK_FAST_MAX_THREADS threads, at least that many of them
+// resident per SM. Two nodes per thread: 64 x 8 gives D3Q19 / D3Q27 128 registers (16 warps per SM), which their 38 / 54
+// loads in flight need without spills. Sphere channel FP32 256x128x128, 160^3, 48^3: 108.5, 108.9, 6.8 us a step; at
+// 96 registers (20 warps) 119.1, 120.1, 9.0. D2Q9 carries half the values: 64 registers and 32 warps (2048x1024:
+// 22.0 us, 25.1 with 96 registers); 96 where a batch's arguments have to be read (60 channels: 56.2 -> 52.2 us).
 #ifndef WK_FAST_MAX_THREADS
 #define WK_FAST_MAX_THREADS 64
 #endif
-#ifndef WK_FAST_TRT_MIN_BLOCKS
-#define WK_FAST_TRT_MIN_BLOCKS 10
+#ifndef WK_PAIRS_MIN_BLOCKS
+#define WK_PAIRS_MIN_BLOCKS 8
 #endif
-#ifndef WK_FAST_OTHER_MIN_BLOCKS
-#define WK_FAST_OTHER_MIN_BLOCKS 8
+#ifndef WK_PAIRS9_MIN_BLOCKS
+#define WK_PAIRS9_MIN_BLOCKS 16
 #endif
-// D2Q9 TRT carries nine populations per node, half of D3Q19's: at 16 blocks per SM it fits 64
-// registers without spills, twice the resident warps, which its fewer loads per thread need to
-// keep enough bytes in flight.
-#ifndef WK_FAST_TRT9_MIN_BLOCKS
-#define WK_FAST_TRT9_MIN_BLOCKS 16
+#ifndef WK_PAIRS9_BATCH_MIN_BLOCKS
+#define WK_PAIRS9_BATCH_MIN_BLOCKS 12
 #endif
 
 namespace wk {

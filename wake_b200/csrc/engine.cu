@@ -39,16 +39,16 @@ void clear_error() {
     t_code = 0;
 }
 
-cudaError_t launch_step_any(int Q, int coll, int store, bool les, const StepArgs& a, const Launch& L, bool fast) {
-    if (Q == 9) return launch_step_q9(coll, store, les, a, L, fast);
-    if (Q == 19) return launch_step_q19(coll, store, les, a, L, fast);
-    return launch_step_q27(coll, store, les, a, L, fast);
+cudaError_t launch_cells_any(int Q, int coll, int store, bool les, const StepArgs& a, int tpb, cudaStream_t stream) {
+    if (Q == 9) return launch_cells_q9(coll, store, les, a, tpb, stream);
+    if (Q == 19) return launch_cells_q19(coll, store, les, a, tpb, stream);
+    return launch_cells_q27(coll, store, les, a, tpb, stream);
 }
-cudaError_t launch_batch_any(int Q, int coll, int store, bool les, const BatchArgs& b, int tpb, cudaStream_t stream,
-                             bool fast, bool idx32) {
-    if (Q == 9) return launch_batch_q9(coll, store, les, b, tpb, stream, fast, idx32);
-    if (Q == 19) return launch_batch_q19(coll, store, les, b, tpb, stream, fast, idx32);
-    return launch_batch_q27(coll, store, les, b, tpb, stream, fast, idx32);
+cudaError_t launch_batch_any(int Q, int coll, int store, bool les, const BatchArgs& b, bool thermal, int tpb,
+                             cudaStream_t stream) {
+    if (Q == 9) return launch_batch_q9(coll, store, les, b, thermal, tpb, stream);
+    if (Q == 19) return launch_batch_q19(coll, store, les, b, thermal, tpb, stream);
+    return launch_batch_q27(coll, store, les, b, thermal, tpb, stream);
 }
 cudaError_t launch_tiles_any(int Q, int coll, int store, bool les, const StepArgs& a, const TileArgs& t,
                              cudaStream_t stream) {
@@ -86,11 +86,11 @@ cudaError_t launch_flags_any(int Q, const uint8_t* types, uint8_t* flags, const 
     if (Q == 19) return launch_flags_q19(types, flags, geo, cfg, L);
     return launch_flags_q27(types, flags, geo, cfg, L);
 }
-cudaError_t launch_seg_class_any(int Q, const uint8_t* flags, uint8_t* cls, const Geo& geo, long long nsegs,
-                                 cudaStream_t stream) {
-    if (Q == 9) return launch_seg_class_q9(flags, cls, geo, nsegs, stream);
-    if (Q == 19) return launch_seg_class_q19(flags, cls, geo, nsegs, stream);
-    return launch_seg_class_q27(flags, cls, geo, nsegs, stream);
+cudaError_t launch_records_any(int Q, const uint8_t* flags, uint4* list, unsigned n, unsigned general, uint4* records,
+                               const Links& links, const Geo& geo, const FlagCfg& cfg, cudaStream_t stream) {
+    if (Q == 9) return launch_records_q9(flags, list, n, general, records, links, geo, cfg, stream);
+    if (Q == 19) return launch_records_q19(flags, list, n, general, records, links, geo, cfg, stream);
+    return launch_records_q27(flags, list, n, general, records, links, geo, cfg, stream);
 }
 
 // ---------------------------------------------------------------- small kernels
@@ -166,6 +166,33 @@ __global__ void k_row_kind(const uint8_t* __restrict__ flags, uint8_t* __restric
                        : static_cast<uint8_t>(0);
 }
 
+// Kind of every segment (cells.cuh), one warp per segment.
+__global__ void k_seg_kind(const uint8_t* __restrict__ flags, uint8_t* __restrict__ seg, int nx, int nseg, long long segs) {
+    const long long e = blockIdx.x * static_cast<long long>(blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (e >= segs) return;
+    const int x0 = static_cast<int>(e % nseg) * CELL;
+    bool pure = true, solid = true;
+    for (int x = x0 + static_cast<int>(threadIdx.x & 31); x < min(nx, x0 + CELL); x += 32) {
+        const uint8_t fl = flags[e / nseg * nx + x];
+        pure = pure && (fl & FL_FAST);
+        solid = solid && (fl & FL_TYPE) == CT_SOLID;
+    }
+    pure = __all_sync(0xffffffffu, pure);
+    solid = __all_sync(0xffffffffu, solid);
+    if ((threadIdx.x & 31) == 0) seg[e] = pure ? wk::SEG_PURE : (solid ? wk::SEG_SOLID : wk::SEG_GENERAL);
+}
+
+// CELL_ZH of every linear cell (cells.cuh), one warp per cell.
+__global__ void k_cell_zh(const uint8_t* __restrict__ flags, uint8_t* __restrict__ kind, long long nodes, long long ncells) {
+    const long long c = blockIdx.x * static_cast<long long>(blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (c >= ncells) return;
+    bool zh = false;
+    for (long long i = c * CELL + (threadIdx.x & 31); i < min(nodes, (c + 1) * CELL); i += 32)
+        zh = zh || (flags[i] & (FL_ZH_IN | FL_ZH_OUT));
+    zh = __any_sync(0xffffffffu, zh);
+    if ((threadIdx.x & 31) == 0) kind[c] = zh ? wk::CELL_ZH : 0;
+}
+
 // Deterministic per-block partial sums for the diagnostics:
 // [0] mass over Fluid, [1] kinetic energy over Fluid, [2] max speed over Fluid,
 // [3] mass over every non-solid cell.
@@ -201,13 +228,11 @@ __global__ void k_diag_partials(const float* __restrict__ rho, const float* __re
         for (int c = 0; c < 4; ++c) part[4 * blockIdx.x + c] = s[c][0];
 }
 
-// Sum the per-node momentum-exchange contributions of one step in slot order
-// (one block: thread t takes slots t, t + 256, ... in order, then a fixed tree)
-// and append the force to the history. Launched after the step kernel that
-// wrote the slots, on the same stream.
-__global__ void __launch_bounds__(256) k_mem_reduce(const double* __restrict__ contrib, int n, unsigned* hist_step,
-                                                    double* hist, int hist_cap) {
-    mem_reduce_block(contrib, n, hist_step, hist, hist_cap);
+// The outstanding force of the last step (if any), when the host wants it or its slots are about to change.
+__global__ void k_mem_flush(const MemCfg mem) {
+    mem_sum(mem);
+    __syncwarp();
+    if (threadIdx.x == 0) *mem.pending = 0u;
 }
 
 // ---------------------------------------------------------------- device initialisation
@@ -380,7 +405,19 @@ int rasterise(wake_grid* g, const wk::RasterBox& b, const wk::RasterShape& sh) {
     return WAKE_OK;
 }
 
-// Upload types and links, rebuild flags and momentum-exchange slots.
+FlagCfg flag_cfg(const wake_grid* g) {
+    FlagCfg cfg{};
+    cfg.zh_rule = (g->Q == 9) ? 1 : 2;
+    cfg.inflow = g->inflow;
+    cfg.outflow = g->outflow;
+    cfg.mem_enabled = g->mem_on;
+    for (int a = 0; a < 3; ++a) cfg.center[a] = g->center[a];
+    cfg.r_max = g->rmax;
+    cfg.r_max_sq = g->rmax * g->rmax;
+    return cfg;
+}
+
+// Upload types and links, rebuild the flags; the step lists follow when a step needs them.
 int rebuild_flags(wake_grid* g) {
     if (g->links_dirty) {
         const int r = upload_links(g);
@@ -391,14 +428,7 @@ int rebuild_flags(wake_grid* g) {
         const int r = dev_types(g);
         if (r) return r;
     }
-    FlagCfg cfg{};
-    cfg.zh_rule = (g->Q == 9) ? 1 : 2;
-    cfg.inflow = g->inflow;
-    cfg.outflow = g->outflow;
-    cfg.mem_enabled = g->mem_on;
-    for (int a = 0; a < 3; ++a) cfg.center[a] = g->center[a];
-    cfg.r_max = g->rmax;
-    cfg.r_max_sq = g->rmax * g->rmax;
+    const FlagCfg cfg = flag_cfg(g);
     const Geo geo = g->geo();
     WK_CUDA(launch_flags_any(g->Q, g->d_types.as<uint8_t>(), g->d_flags.as<uint8_t>(), geo, cfg, g->launch()));
     const int nl = g->dev_links;
@@ -408,197 +438,286 @@ int rebuild_flags(wake_grid* g) {
         WK_CUDA(launch_link_marks(g->d_link_node.as<int>(), nl, g->d_flags.as<uint8_t>(), g->d_nodestart.as<int>(),
                                   g->stream));
     }
-    // split the rows into SEG-node segments for the two step kernels
-    {
-        const int nseg = (g->nx + SEG - 1) / SEG;
-        const long long nsegs = static_cast<long long>(g->rows) * nseg;
-        if (nsegs >= (1ll << 32)) return set_error(WAKE_ERR_INVALID, "lattice too large for 32-bit segment numbers");
-        DevMem cls;
-        WK_CUDA(cls.ensure(static_cast<std::size_t>(nsegs)));
-        WK_CUDA(launch_seg_class_any(g->Q, g->d_flags.as<uint8_t>(), cls.as<uint8_t>(), geo, nsegs, g->stream));
-        std::vector<uint8_t> h(static_cast<std::size_t>(nsegs));
-        WK_CUDA(cudaMemcpyAsync(h.data(), cls.p, h.size(), cudaMemcpyDeviceToHost, g->stream));
-        WK_CUDA(cudaStreamSynchronize(g->stream));
-        cls.release();
-        // general segments; pure-gather spans: whole rows, or the runs of pure-gather
-        // segments of the rows that hold general segments
-        if (g->th.on)  // the coupled temperature runs on the general per-node path only
-            for (auto& c : h) c = static_cast<uint8_t>(c & ~1u);
-        std::vector<unsigned> gen;
-        std::vector<uint4> spans, mixed_spans;
-        std::vector<uint8_t> row_fast(static_cast<std::size_t>(g->rows), 1);
-        for (long long e = 0; e < nsegs; ++e) {
-            if (h[e] & 1) continue;
-            row_fast[static_cast<std::size_t>(e / nseg)] = 0;
-            if (h[e] & 4) continue;  // every node solid: frozen in both buffers, nothing to launch
-            gen.push_back(static_cast<unsigned>(e));
-        }
-        for (int r = 0; r < g->rows; ++r) {
-            if (row_fast[r]) {
-                spans.push_back(make_uint4(0u, static_cast<unsigned>(r), 0u, static_cast<unsigned>(g->nx)));
-                continue;
-            }
-            for (int sg = 0; sg < nseg;) {
-                if (!(h[static_cast<long long>(r) * nseg + sg] & 1)) {
-                    ++sg;
-                    continue;
-                }
-                int s1 = sg + 1;
-                while (s1 < nseg && (h[static_cast<long long>(r) * nseg + s1] & 1)) ++s1;
-                const uint4 sp = make_uint4(0u, static_cast<unsigned>(r), static_cast<unsigned>(sg * SEG),
-                                            static_cast<unsigned>(std::min(g->nx, s1 * SEG)));
-                spans.push_back(sp);
-                mixed_spans.push_back(sp);
-                sg = s1;
-            }
-        }
-        g->n_fast = static_cast<int>(spans.size());
-        g->n_gen = static_cast<int>(gen.size());
-        WK_CUDA(g->d_fast_rows.ensure(sizeof(uint4) * std::max<std::size_t>(1, spans.size())));
-        WK_CUDA(g->d_gen_rows.ensure(sizeof(unsigned) * std::max<std::size_t>(1, gen.size())));
-        if (!spans.empty())
-            WK_CUDA(cudaMemcpyAsync(g->d_fast_rows.p, spans.data(), sizeof(uint4) * spans.size(),
-                                    cudaMemcpyHostToDevice, g->stream));
-        if (!gen.empty())
-            WK_CUDA(cudaMemcpyAsync(g->d_gen_rows.p, gen.data(), sizeof(unsigned) * gen.size(), cudaMemcpyHostToDevice,
-                                    g->stream));
-        // momentum-exchange slots: per general segment and 32-node chunk, the number of
-        // FL_MEM nodes before it (node order), so slots are dense and ordered
-        g->warps_per_row = SEG / 32;
-        g->n_mem_nodes = 0;
-        std::vector<int> warp_base;
-        if (g->mem_on) {
-            std::vector<uint8_t> fl(g->N);
-            WK_CUDA(cudaMemcpyAsync(fl.data(), g->d_flags.p, g->N, cudaMemcpyDeviceToHost, g->stream));
-            WK_CUDA(cudaStreamSynchronize(g->stream));
-            warp_base.assign(std::max<std::size_t>(1, gen.size() * g->warps_per_row), 0);
-            int count = 0;
-            for (std::size_t k = 0; k < gen.size(); ++k) {
-                const long long row = gen[k] / nseg, x0 = (gen[k] % nseg) * SEG;
-                for (int c = 0; c < g->warps_per_row; ++c) {
-                    warp_base[k * g->warps_per_row + c] = count;
-                    const long long xa = x0 + 32 * c, xe = std::min<long long>(g->nx, xa + 32);
-                    for (long long x = xa; x < xe; ++x) count += (fl[row * g->nx + x] & FL_MEM) ? 1 : 0;
-                }
-            }
-            g->n_mem_nodes = count;
-            WK_CUDA(g->d_warp_base.ensure(sizeof(int) * warp_base.size()));
-            WK_CUDA(cudaMemcpyAsync(g->d_warp_base.p, warp_base.data(), sizeof(int) * warp_base.size(),
-                                    cudaMemcpyHostToDevice, g->stream));
-            WK_CUDA(g->d_contrib.ensure(sizeof(double) * 3 * std::max(1, count)));
-        }
-        // persistent-kernel work: tiles of consecutive all-pure-gather rows of one z plane
-        // (at most TILE_NODES nodes), the general segments with their slot entry, and the
-        // pure-gather runs of the other rows
-        {
-            const int per_tile = std::max(1, TILE_NODES / g->nx);
-            std::vector<uint4> tiles, gen4;
-            for (int r = 0; r < g->rows;) {
-                if (!row_fast[r]) {
-                    ++r;
-                    continue;
-                }
-                const int z = r / g->ny, y0 = r % g->ny;
-                int cnt = 1;
-                while (cnt < per_tile && r + cnt < g->rows && row_fast[r + cnt] && (r + cnt) / g->ny == z) ++cnt;
-                tiles.push_back(make_uint4(0u, (static_cast<unsigned>(z) << 16) | static_cast<unsigned>(y0),
-                                           static_cast<unsigned>(cnt), 0u));
-                r += cnt;
-            }
-            for (std::size_t k = 0; k < gen.size(); ++k)
-                gen4.push_back(make_uint4(0u, gen[k], static_cast<unsigned>(k), 0u));
-            WK_CUDA(g->d_tiles.ensure(sizeof(uint4) * std::max<std::size_t>(1, tiles.size())));
-            WK_CUDA(g->d_gen4.ensure(sizeof(uint4) * std::max<std::size_t>(1, gen4.size())));
-            WK_CUDA(g->d_mixed.ensure(sizeof(uint4) * std::max<std::size_t>(1, mixed_spans.size())));
-            if (!tiles.empty())
-                WK_CUDA(cudaMemcpyAsync(g->d_tiles.p, tiles.data(), sizeof(uint4) * tiles.size(), cudaMemcpyHostToDevice,
-                                        g->stream));
-            if (!gen4.empty())
-                WK_CUDA(cudaMemcpyAsync(g->d_gen4.p, gen4.data(), sizeof(uint4) * gen4.size(), cudaMemcpyHostToDevice,
-                                        g->stream));
-            if (!mixed_spans.empty())
-                WK_CUDA(cudaMemcpyAsync(g->d_mixed.p, mixed_spans.data(), sizeof(uint4) * mixed_spans.size(),
-                                        cudaMemcpyHostToDevice, g->stream));
-            WK_CUDA(cudaStreamSynchronize(g->stream));  // the host vectors go out of scope
-            g->n_tiles = static_cast<int>(tiles.size());
-            g->n_tile_gen = static_cast<int>(gen4.size());
-            g->n_mixed = static_cast<int>(mixed_spans.size());
-            g->h_tiles = std::move(tiles);
-            g->h_gen4 = std::move(gen4);
-            g->h_mixed = std::move(mixed_spans);
-        }
-        // whole-row kernel: one descriptor byte per row (rows.cuh), kept only where it agrees
-        // with the segment classes (ROW_FAST exactly on the rows whose segments are all pure)
-        {
-            WK_CUDA(g->d_row_kind.ensure(static_cast<std::size_t>(g->rows)));
-            const int rows_per_block = 8;
-            k_row_kind<<<(g->rows + rows_per_block - 1) / rows_per_block, 32 * rows_per_block, 0, g->stream>>>(
-                g->d_flags.as<uint8_t>(), g->d_row_kind.as<uint8_t>(), g->nx, g->rows);
-            WK_CUDA(cudaGetLastError());
-            std::vector<uint8_t> kinds(static_cast<std::size_t>(g->rows));
-            WK_CUDA(cudaMemcpyAsync(kinds.data(), g->d_row_kind.p, kinds.size(), cudaMemcpyDeviceToHost, g->stream));
-            WK_CUDA(cudaStreamSynchronize(g->stream));
-            int n_rf = 0;
-            bool agree = true;
-            for (int r = 0; r < g->rows; ++r) {
-                const bool k = (kinds[r] & wk::ROW_FAST) != 0;
-                agree = agree && (k == (row_fast[r] != 0));
-                n_rf += k ? 1 : 0;
-            }
-            g->n_row_fast = agree ? n_rf : 0;
-            g->row_fast_nodes = static_cast<long long>(g->n_row_fast) * g->nx;
-            std::vector<unsigned> list;
-            if (g->n_row_fast > 0 && g->rows < (1 << 28)) {
-                list.reserve(static_cast<std::size_t>(g->n_row_fast));
-                for (int r = 0; r < g->rows; ++r)
-                    if (kinds[r] & wk::ROW_FAST) list.push_back(static_cast<unsigned>(r) | (unsigned(kinds[r]) << 28));
-                WK_CUDA(g->d_row_list.ensure(sizeof(unsigned) * list.size()));
-                WK_CUDA(cudaMemcpyAsync(g->d_row_list.p, list.data(), sizeof(unsigned) * list.size(),
-                                        cudaMemcpyHostToDevice, g->stream));
-                WK_CUDA(cudaStreamSynchronize(g->stream));  // the host list goes out of scope
-            }
-        }
-        g->h_fast_rows = std::move(spans);
-        g->h_gen_rows = std::move(gen);
-    }
     g->geom_version = next_geom_version();
     g->geom_dirty = false;
     g->invalidate_graph();
     return WAKE_OK;
 }
 
-// Upload the links (sorted by fluid node) and their moving-wall terms.
+// Append the last step's outstanding force.
+int flush_force(wake_grid* g) {
+    if (!g->mem_on || g->mem_list == 0 || !(g->mem_left || g->mem_captured)) return WAKE_OK;
+    const StepArgs a = wk::grid_step_args(g, g->mem_list == 2);
+    k_mem_flush<<<1, 32, 0, g->stream>>>(a.mem);
+    WK_CUDA(cudaGetLastError());
+    g->mem_left = false;
+    return WAKE_OK;
+}
+
+// The cells of consecutive segments of one kind, as a list: nodes [begin, end), cut every CELL nodes from the start
+// (a shorter first cell where that is odd: a 16-bit pair is stored as one word at even nodes).
+void list_run(std::vector<uint4>& list, long long begin, long long end, bool pure) {
+    for (long long i = begin; i < end;) {
+        const long long next = std::min(end, i + CELL - (pure ? i & 1 : 0));
+        list.push_back(make_uint4(static_cast<unsigned>(i), static_cast<unsigned>(next - i), 0u, 0u));
+        i = next;
+    }
+}
+
+// Calls run(begin, end, kind) for the longest runs of SEG_GENERAL and of SEG_PURE segments in the node order;
+// rows with skip[row] & ROW_FAST are left out.
+template <class Run>
+void for_runs(const wake_grid* g, const uint8_t* skip, Run run) {
+    const int nseg = (g->nx + CELL - 1) / CELL;
+    uint8_t kind = wk::SEG_SOLID;  // of the open run: none
+    long long begin = 0;
+    for (int row = 0; row < g->rows; ++row)
+        for (int k = 0; k < nseg; ++k) {
+            const uint8_t now = skip && (skip[row] & wk::ROW_FAST) ? static_cast<uint8_t>(wk::SEG_SOLID)
+                                                                   : g->h_seg[static_cast<std::size_t>(row) * nseg + k];
+            if (now == kind) continue;
+            const long long i = static_cast<long long>(row) * g->nx + k * CELL;
+            if (kind != wk::SEG_SOLID) run(begin, i, kind);
+            kind = now;
+            begin = i;
+        }
+    if (kind != wk::SEG_SOLID) run(begin, g->N, kind);
+}
+
+// Device list of cells with their node records, for the current flags.
+int build_list(wake_grid* g, wk::CellList& L, const std::vector<uint4>& general, const std::vector<uint4>& pure) {
+    const int rf = flush_force(g);  // its slots may be this list's
+    if (rf) return rf;
+    L.general = static_cast<unsigned>(general.size());
+    L.cells = general;
+    L.cells.insert(L.cells.end(), pure.begin(), pure.end());
+    // the curved links of each cell: a run of the node-ordered link array
+    std::size_t k = 0;
+    for (unsigned e = 0; e < L.general; ++e) {
+        uint4& c = L.cells[e];
+        while (k < g->dev_link_node.size() && static_cast<unsigned>(g->dev_link_node[k]) < c.x) ++k;
+        std::size_t last = k;
+        while (last < g->dev_link_node.size() && static_cast<unsigned>(g->dev_link_node[last]) < c.x + c.y) ++last;
+        c.z = static_cast<unsigned>(k);
+        c.w = static_cast<unsigned>(last - k);
+        k = last;
+    }
+    WK_CUDA(L.list.ensure(sizeof(uint4) * std::max<std::size_t>(1, L.cells.size())));
+    WK_CUDA(L.records.ensure(sizeof(uint4) * CELL * std::max(1u, L.general)));
+    if (!L.cells.empty()) {
+        const std::size_t bytes = sizeof(uint4) * L.cells.size();
+        WK_CUDA(cudaMemcpyAsync(L.list.p, L.cells.data(), bytes, cudaMemcpyHostToDevice, g->stream));
+        WK_CUDA(launch_records_any(g->Q, g->d_flags.as<uint8_t>(), L.list.as<uint4>(), static_cast<unsigned>(L.cells.size()),
+                                   L.general, L.records.as<uint4>(), g->links(), g->geo(), flag_cfg(g), g->stream));
+        WK_CUDA(cudaMemcpyAsync(L.cells.data(), L.list.p, bytes, cudaMemcpyDeviceToHost, g->stream));  // with the LIST_* bits
+    }
+    WK_CUDA(cudaStreamSynchronize(g->stream));
+    L.mode = 0;
+    L.version = g->geom_version;
+    return WAKE_OK;
+}
+
+// Units of a list's cells and their momentum-exchange slots, for the grid's current model.
+int ensure_units(wake_grid* g, wk::CellList& L) {
+    const bool pairs3 = g->storage == WAKE_STORE_F32 && g->Q != 9;  // all_pairs, pure_pairs (pairs2.cuh)
+    const bool whole = !g->th.on && g->collision != WAKE_TRT && pairs3;
+    const bool pure_whole = !g->th.on && (g->collision == WAKE_TRT || pairs3);
+    const int mode = 1 + (whole ? 1 : 0) + (pure_whole ? 2 : 0);
+    if (L.mode == mode) return WAKE_OK;
+    const int rf = flush_force(g);  // the outstanding force is in the old slots
+    if (rf) return rf;
+    const unsigned n = static_cast<unsigned>(L.cells.size());
+    std::vector<int> slot(2 * static_cast<std::size_t>(L.general), 0);
+    L.units.clear();
+    L.slots = 0;
+    for (unsigned e = 0; e < L.general; ++e) {
+        const unsigned b = L.cells[e].y;
+        for (unsigned h = 0; h < (whole ? 1u : 2u); ++h) {
+            const unsigned halves = whole ? 3u : 1u << h;
+            if (b & (wk::LIST_LIVE * halves)) L.units.push_back(4 * e + h);
+            slot[2 * e + h] = L.slots;
+            if (b & (wk::LIST_MEM * halves)) ++L.slots;
+        }
+    }
+    for (unsigned e = L.general; e < n; ++e)
+        for (unsigned h = 0; h < (pure_whole || (L.cells[e].y & 0xffu) <= CELL / 2 ? 1u : 2u); ++h)
+            L.units.push_back(4 * e + wk::UNIT_PURE + h);
+    WK_CUDA(L.d_units.ensure(sizeof(unsigned) * std::max<std::size_t>(1, L.units.size())));
+    WK_CUDA(L.slot.ensure(sizeof(int) * std::max<std::size_t>(1, slot.size())));
+    L.stride = 3ll * std::max(1, L.slots);
+    if (g->mem_on) WK_CUDA(L.contrib.ensure(sizeof(double) * 2 * static_cast<std::size_t>(L.stride)));
+    if (!L.units.empty())
+        WK_CUDA(cudaMemcpyAsync(L.d_units.p, L.units.data(), sizeof(unsigned) * L.units.size(), cudaMemcpyHostToDevice,
+                                g->stream));
+    if (!slot.empty())
+        WK_CUDA(cudaMemcpyAsync(L.slot.p, slot.data(), sizeof(int) * slot.size(), cudaMemcpyHostToDevice, g->stream));
+    WK_CUDA(cudaStreamSynchronize(g->stream));  // the host list goes out of scope
+    L.mode = mode;
+    g->units_version = wk::next_geom_version();
+    g->invalidate_graph();
+    return WAKE_OK;
+}
+
+// Queue the kinds of the segments and their copy to h_seg.
+int queue_segments(wake_grid* g) {
+    if (g->seg_version == g->geom_version) return WAKE_OK;
+    const int nseg = (g->nx + CELL - 1) / CELL;
+    const long long segs = static_cast<long long>(g->rows) * nseg;
+    WK_CUDA(g->d_seg.ensure(static_cast<std::size_t>(segs)));
+    g->h_seg.resize(static_cast<std::size_t>(segs));
+    k_seg_kind<<<static_cast<unsigned>((segs + 7) / 8), 256, 0, g->stream>>>(g->d_flags.as<uint8_t>(),
+                                                                            g->d_seg.as<uint8_t>(), g->nx, nseg, segs);
+    WK_CUDA(cudaGetLastError());
+    WK_CUDA(cudaMemcpyAsync(g->h_seg.data(), g->d_seg.p, g->h_seg.size(), cudaMemcpyDeviceToHost, g->stream));
+    g->seg_version = g->geom_version;
+    return WAKE_OK;
+}
+
+// Linear and listed cells of the whole lattice.
+int ensure_cells(wake_grid* g) {
+    if (g->cells.version == g->geom_version) return WAKE_OK;
+    const int rs = queue_segments(g);
+    if (rs) return rs;
+    const long long ncells = (g->N + CELL - 1) / CELL;
+    WK_CUDA(g->d_kind.ensure(static_cast<std::size_t>(ncells)));
+    k_cell_zh<<<static_cast<unsigned>((ncells + 7) / 8), 256, 0, g->stream>>>(g->d_flags.as<uint8_t>(),
+                                                                             g->d_kind.as<uint8_t>(), g->N, ncells);
+    WK_CUDA(cudaGetLastError());
+    g->h_kind.resize(static_cast<std::size_t>(ncells));
+    WK_CUDA(cudaMemcpyAsync(g->h_kind.data(), g->d_kind.p, g->h_kind.size(), cudaMemcpyDeviceToHost, g->stream));
+    WK_CUDA(cudaStreamSynchronize(g->stream));
+    std::vector<uint4> general, pure;
+    g->cell_nodes = 0;
+    for_runs(g, nullptr, [&](long long begin, long long end, uint8_t kind) {
+        g->cell_nodes += end - begin;
+        if (kind == wk::SEG_GENERAL) {
+            list_run(general, begin, end, false);
+            return;
+        }
+        // Linear cells, and the ends that they leave as listed ones; a short run is listed whole where that makes
+        // fewer cells (200 nodes: 4 instead of 3 linear ones and 2 ends). A listed cell costs two more
+        // dependent loads, so a long run stays linear.
+        const long long first = (begin + CELL - 1) / CELL, last = end == g->N ? ncells : end / CELL;
+        const long long ends = (begin % CELL != 0) + (last * CELL < end);
+        if (last <= first || (last - first < 16 && (end - begin + (begin & 1) + CELL - 1) / CELL < last - first + ends)) {
+            list_run(pure, begin, end, true);
+            return;
+        }
+        list_run(pure, begin, first * CELL, true);
+        for (long long c = first; c < last; ++c) g->h_kind[static_cast<std::size_t>(c)] |= wk::CELL_PURE;
+        list_run(pure, last * CELL, end, true);
+    });
+    WK_CUDA(cudaMemcpyAsync(g->d_kind.p, g->h_kind.data(), g->h_kind.size(), cudaMemcpyHostToDevice, g->stream));
+    return build_list(g, g->cells, general, pure);
+}
+
+// Row tables of the bulk kernels (variants 2 to 4) and the cells of the other rows.
+int ensure_rows(wake_grid* g) {
+    if (g->rest.version == g->geom_version) return WAKE_OK;
+    const int rs = queue_segments(g);
+    if (rs) return rs;
+    WK_CUDA(g->d_row_kind.ensure(static_cast<std::size_t>(g->rows)));
+    k_row_kind<<<(g->rows + 7) / 8, 256, 0, g->stream>>>(g->d_flags.as<uint8_t>(), g->d_row_kind.as<uint8_t>(), g->nx,
+                                                         g->rows);
+    WK_CUDA(cudaGetLastError());
+    std::vector<uint8_t> kinds(static_cast<std::size_t>(g->rows));
+    WK_CUDA(cudaMemcpyAsync(kinds.data(), g->d_row_kind.p, kinds.size(), cudaMemcpyDeviceToHost, g->stream));
+    WK_CUDA(cudaStreamSynchronize(g->stream));
+    std::vector<uint4> general, pure;
+    for_runs(g, kinds.data(), [&](long long begin, long long end, uint8_t kind) {
+        list_run(kind == wk::SEG_GENERAL ? general : pure, begin, end, kind != wk::SEG_GENERAL);
+    });
+    std::vector<unsigned> fast;
+    std::vector<uint4> tiles;
+    const int per_tile = std::max(1, TILE_NODES / g->nx);
+    for (int r = 0; r < g->rows; ++r) {
+        if (!(kinds[r] & wk::ROW_FAST)) continue;
+        fast.push_back(static_cast<unsigned>(r) | (static_cast<unsigned>(kinds[r]) << 28));
+        // a tile takes up to per_tile consecutive rows of one z plane
+        const unsigned zy = (static_cast<unsigned>(r / g->ny) << 16) | static_cast<unsigned>(r % g->ny);
+        if (!tiles.empty() && r % g->ny && tiles.back().y + tiles.back().z == zy &&
+            tiles.back().z < static_cast<unsigned>(per_tile))
+            ++tiles.back().z;
+        else
+            tiles.push_back(make_uint4(0u, zy, 1u, 0u));
+    }
+    g->n_row_fast = static_cast<int>(fast.size());
+    g->n_tiles = static_cast<int>(tiles.size());
+    WK_CUDA(g->d_row_list.ensure(sizeof(unsigned) * std::max<std::size_t>(1, fast.size())));
+    WK_CUDA(g->d_tiles.ensure(sizeof(uint4) * std::max<std::size_t>(1, tiles.size())));
+    if (!fast.empty()) {
+        WK_CUDA(cudaMemcpyAsync(g->d_row_list.p, fast.data(), sizeof(unsigned) * fast.size(), cudaMemcpyHostToDevice,
+                                g->stream));
+        WK_CUDA(cudaMemcpyAsync(g->d_tiles.p, tiles.data(), sizeof(uint4) * tiles.size(), cudaMemcpyHostToDevice,
+                                g->stream));
+    }
+    return build_list(g, g->rest, general, pure);  // synchronises: the host tables go out of scope
+}
+
+// The lists that the next step's kernels read.
+int ensure_lists(wake_grid* g) {
+    if (g->tiles_fit() || g->rows_fit() || g->pipe_fits()) {
+        const int r = ensure_rows(g);
+        if (r) return r;
+        if (g->by_rows()) return ensure_units(g, g->rest);
+    }
+    const int r = ensure_cells(g);
+    return r ? r : ensure_units(g, g->cells);
+}
+
+// Upload the links, sorted by fluid node and replaced direction, and their moving-wall terms. Of links that
+// replace the same population the last one given counts.
 int upload_links(wake_grid* g) {
-    const int n = static_cast<int>(g->link_node.size());
+    const int given = static_cast<int>(g->link_node.size());
     g->dev_links = 0;
-    if (n == 0) return WAKE_OK;
-    std::vector<int> order(n);
+    g->dev_link_node.clear();
+    if (given == 0) return WAKE_OK;
+    std::vector<int> order(given);
     std::iota(order.begin(), order.end(), 0);
-    std::stable_sort(order.begin(), order.end(),
-                     [&](int a, int b) { return g->link_node[a] < g->link_node[b]; });
-    std::vector<int> node(n), q(n);
-    std::vector<float> delta(n), mom(n);
+    auto key = [&](int k) { return static_cast<long long>(g->link_node[k]) * 32 + g->lat.opp[g->link_q[k]]; };
+    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return key(a) < key(b); });
+    int n = 0;
+    for (int j = 0; j < given; ++j)
+        if (j + 1 == given || key(order[j + 1]) != key(order[j])) order[n++] = order[j];
+    std::vector<int> node(n);
+    std::vector<uint4> rec(n);
+    std::vector<float> mom(n);
     for (int j = 0; j < n; ++j) {
-        const int k = order[j];
-        node[j] = g->link_node[k];
-        q[j] = g->link_q[k];
-        delta[j] = g->link_delta[k];
-        const int qq = q[j];
-        const float ci_uw = float(g->lat.cx[qq]) * g->link_uw[3 * k] + float(g->lat.cy[qq]) * g->link_uw[3 * k + 1] +
-                            float(g->lat.cz[qq]) * g->link_uw[3 * k + 2];
-        // d3q19_curved.ispc:57 (delta < 1/2) and :62 (delta >= 1/2)
-        mom[j] = (delta[j] < 0.5f) ? 2.0f * g->lat.w[qq] * 1.0f * 3.0f * ci_uw
-                                   : (1.0f / delta[j]) * g->lat.w[qq] * 1.0f * 3.0f * ci_uw;
+        const int k = order[j], i = g->link_node[k], q = g->link_q[k], o = g->lat.opp[q];
+        const float delta = g->link_delta[k];
+        const float ci_uw = float(g->lat.cx[q]) * g->link_uw[3 * k] + float(g->lat.cy[q]) * g->link_uw[3 * k + 1] +
+                            float(g->lat.cz[q]) * g->link_uw[3 * k + 2];
+        // d3q19_curved.ispc:46-68: delta < 1/2 interpolates between the node and the one behind it (the node
+        // itself where that lies past a y or z face), delta >= 1/2 between the two directions at the node
+        int second = i, plane = q;
+        float c;
+        if (delta < 0.5f) {
+            const int x = i % g->nx, y = (i / g->nx) % g->ny, z = i / (g->nx * g->ny);
+            const int xf = (x - g->lat.cx[q] + g->nx) % g->nx, yf = y - g->lat.cy[q], zf = z - g->lat.cz[q];
+            if (yf >= 0 && yf < g->ny && zf >= 0 && zf < g->nz) second = static_cast<int>(idx3(g, xf, yf, zf));
+            c = 2.0f * delta;
+            mom[j] = 2.0f * g->lat.w[q] * 1.0f * 3.0f * ci_uw;
+        } else {
+            plane = o;
+            c = 1.0f / (2.0f * delta);
+            mom[j] = (1.0f / delta) * g->lat.w[q] * 1.0f * 3.0f * ci_uw;
+        }
+        node[j] = i;
+        unsigned bits;
+        std::memcpy(&bits, &c, sizeof bits);
+        rec[j] = make_uint4(static_cast<unsigned>(i), static_cast<unsigned>(second),
+                            static_cast<unsigned>(q) | (static_cast<unsigned>(plane) << 8) |
+                                (static_cast<unsigned>(o) << 16) | (mom[j] != 0.0f ? wk::LINK_MOVES : 0u),
+                            bits);
     }
     WK_CUDA(g->d_link_node.ensure(sizeof(int) * n));
-    WK_CUDA(g->d_link_q.ensure(sizeof(int) * n));
-    WK_CUDA(g->d_link_delta.ensure(sizeof(float) * n));
+    WK_CUDA(g->d_link_rec.ensure(sizeof(uint4) * n));
     WK_CUDA(g->d_link_mom.ensure(sizeof(float) * n));
     WK_CUDA(cudaMemcpyAsync(g->d_link_node.p, node.data(), sizeof(int) * n, cudaMemcpyHostToDevice, g->stream));
-    WK_CUDA(cudaMemcpyAsync(g->d_link_q.p, q.data(), sizeof(int) * n, cudaMemcpyHostToDevice, g->stream));
-    WK_CUDA(cudaMemcpyAsync(g->d_link_delta.p, delta.data(), sizeof(float) * n, cudaMemcpyHostToDevice, g->stream));
+    WK_CUDA(cudaMemcpyAsync(g->d_link_rec.p, rec.data(), sizeof(uint4) * n, cudaMemcpyHostToDevice, g->stream));
     WK_CUDA(cudaMemcpyAsync(g->d_link_mom.p, mom.data(), sizeof(float) * n, cudaMemcpyHostToDevice, g->stream));
     WK_CUDA(cudaStreamSynchronize(g->stream));
+    g->dev_link_node = std::move(node);
     g->dev_links = n;
     return WAKE_OK;
 }
@@ -708,7 +827,7 @@ int apply_geometry(wake_grid* g) {
     return WAKE_OK;
 }
 
-int prepare(wake_grid* g) {
+int prepare_state(wake_grid* g) {
     const int r = apply_geometry(g);
     if (r) return r;
     if (!g->pending) return WAKE_OK;
@@ -716,7 +835,16 @@ int prepare(wake_grid* g) {
         const int r2 = materialise(g, true, false);
         if (r2) return r2;
     }
+    const int rf = flush_force(g);  // the buffers start over, maybe with another model
+    if (rf) return rf;
     return initial_from_scratch(g);
+}
+
+int prepare(wake_grid* g) {
+    int r = prepare_state(g);
+    if (!r) r = ensure_lists(g);
+    if (!r && g->mem_list != 0 && g->mem_list != (g->by_rows() ? 2 : 1)) r = flush_force(g);  // the other list's slots
+    return r;
 }
 
 // The FP32 scratch now holds f^0: the next step collides it (fresh run, step 0).
@@ -743,94 +871,55 @@ int init_on_device(wake_grid* g, const InitSpec& s) {
     return WAKE_OK;
 }
 
+// Events around a bulk launch when its timing is on.
+int bulk_event(wake_grid* g) {
+    if (!g->time_bulk) return WAKE_OK;
+    if (g->t_ev.size() <= g->t_used) {
+        cudaEvent_t e = nullptr;
+        WK_CUDA(cudaEventCreate(&e));
+        g->t_ev.push_back(e);
+    }
+    WK_CUDA(cudaEventRecord(g->t_ev[g->t_used], g->stream));
+    ++g->t_used;
+    return WAKE_OK;
+}
+
 int do_steps(wake_grid* g, int n) {
+    const bool by_rows = g->by_rows();
+    StepArgs a = wk::grid_step_args(g, by_rows);
     for (int s = 0; s < n; ++s) {
-        StepArgs a = wk::grid_step_args(g);
-        a.fin = g->buf(g->cur);
-        a.fout = g->buf(1 - g->cur);
-        a.th.tin = g->tbuf(g->cur);
-        a.th.tout = g->tbuf(1 - g->cur);
-        if (g->use_tiles()) {
-            // one persistent launch for the general rows and the staged pure-gather tiles,
-            // then the momentum-exchange sum of the slots it wrote
-            const TileArgs t{g->d_tiles.as<uint4>(), g->n_tiles, g->d_gen4.as<uint4>(), g->n_tile_gen, nullptr, 0,
-                             g->d_mixed.as<uint4>(), g->n_mixed};
-            const bool timed = g->time_bulk;
-            if (timed) {
-                while (g->t_ev.size() < g->t_used + 2) {
-                    cudaEvent_t e = nullptr;
-                    WK_CUDA(cudaEventCreate(&e));
-                    g->t_ev.push_back(e);
-                }
-                WK_CUDA(cudaEventRecord(g->t_ev[g->t_used], g->stream));
-            }
-            WK_CUDA(launch_tiles_any(g->Q, g->collision, g->storage, g->les != 0, a, t, g->stream));
-            if (timed) {
-                WK_CUDA(cudaEventRecord(g->t_ev[g->t_used + 1], g->stream));
-                g->t_used += 2;
-            }
-            if (g->mem_on) {
-                k_mem_reduce<<<1, 256, 0, g->stream>>>(a.mem.contrib, a.mem.n_nodes, a.mem.hist_step, a.mem.hist,
-                                                       a.mem.hist_cap);
-                WK_CUDA(cudaGetLastError());
-            }
-            g->cur ^= 1;
-            g->mf_valid = false;
-            for (int c = 0; c < 3; ++c) g->last_step_g[c] = g->phys.g[c];
-            ++g->k;
-            continue;
-        }
-        // The pure-gather rows and the rows with boundaries / momentum exchange write
-        // disjoint nodes of the output, so the small general launch runs on a forked
-        // stream beside the bulk launch (a fork/join that CUDA graph capture keeps).
-        StepArgs gen = a;
-        gen.rows = g->d_gen_rows.as<unsigned>();
-        gen.nrows = g->n_gen;
-        // with the whole-row kernel, the pure-gather runs of the other rows go beside the general segments
-        const bool pipe_k = g->use_pipe();
-        const bool rows_k = pipe_k || g->use_rows();
-        StepArgs part = a;
-        part.spans = g->d_mixed.as<uint4>();
-        part.nspans = rows_k ? g->n_mixed : 0;
-        a.spans = g->d_fast_rows.as<uint4>();
-        a.nspans = rows_k ? 0 : g->n_fast;
-        a.row_kind = g->d_row_kind.as<uint8_t>();
-        const bool bulk = rows_k || g->n_fast > 0;
-        const bool fork = bulk && (g->n_gen > 0 || part.nspans > 0);
-        Launch side = g->launch();
+        wk::grid_step_buffers(g, g->cur, a);
+        // A bulk kernel and the rows beside it write disjoint nodes of the output, so the small launch of
+        // those rows runs on a forked stream (a fork / join that CUDA graph capture keeps). It is issued
+        // first: a persistent bulk kernel fills the device until its end.
+        const bool bulk = by_rows && g->n_row_fast > 0;
+        const bool beside = !by_rows || !g->rest.units.empty() || g->mem_on;
+        const bool fork = bulk && beside;
         if (fork) {
-            side.stream = g->side;
             WK_CUDA(cudaEventRecord(g->ev_fork, g->stream));
             WK_CUDA(cudaStreamWaitEvent(g->side, g->ev_fork, 0));
         }
-        WK_CUDA(launch_step_any(g->Q, g->collision, g->storage, g->les != 0, gen, side, false));
-        if (part.nspans > 0) WK_CUDA(launch_step_any(g->Q, g->collision, g->storage, g->les != 0, part, side, true));
-        if (g->mem_on) {
-            // the step's force from the slots the general launch just wrote (zero if none)
-            k_mem_reduce<<<1, 256, 0, side.stream>>>(a.mem.contrib, a.mem.n_nodes, a.mem.hist_step, a.mem.hist,
-                                                     a.mem.hist_cap);
-            WK_CUDA(cudaGetLastError());
+        if (beside) {
+            int r = by_rows ? WAKE_OK : bulk_event(g);
+            if (r) return r;
+            WK_CUDA(launch_cells_any(g->Q, g->collision, g->storage, g->les != 0, a, g->tpb_cells,
+                                     fork ? g->side : g->stream));
+            if (!by_rows && (r = bulk_event(g))) return r;
         }
-        const bool timed = g->time_bulk && (rows_k || a.nspans > 0);
-        if (timed) {
-            while (g->t_ev.size() < g->t_used + 2) {
-                cudaEvent_t e = nullptr;
-                WK_CUDA(cudaEventCreate(&e));
-                g->t_ev.push_back(e);
+        if (bulk) {
+            int r = bulk_event(g);
+            if (r) return r;
+            if (g->use_tiles()) {
+                const TileArgs t{g->d_tiles.as<uint4>(), g->n_tiles};
+                WK_CUDA(launch_tiles_any(g->Q, g->collision, g->storage, g->les != 0, a, t, g->stream));
+            } else if (g->use_pipe()) {
+                const wk::PipeArgs pa{g->d_row_list.as<unsigned>(), g->n_row_fast};
+                WK_CUDA(launch_rows_pipe_any(g->Q, g->storage, g->les != 0, g->pipe_cap(), a, pa, g->stream));
+            } else {
+                WK_CUDA(launch_rows_any(g->Q, g->storage, g->les != 0, a, g->rows, g->tpb_rows(), g->stream));
             }
-            WK_CUDA(cudaEventRecord(g->t_ev[g->t_used], g->stream));
-        }
-        if (pipe_k) {
-            const wk::PipeArgs pa{g->d_row_list.as<unsigned>(), g->n_row_fast};
-            WK_CUDA(launch_rows_pipe_any(g->Q, g->storage, g->les != 0, g->pipe_cap(), a, pa, g->stream));
-        } else if (rows_k) {
-            WK_CUDA(launch_rows_any(g->Q, g->storage, g->les != 0, a, g->rows, g->tpb_rows(), g->stream));
-        } else {
-            WK_CUDA(launch_step_any(g->Q, g->collision, g->storage, g->les != 0, a, g->launch(), true));
-        }
-        if (timed) {
-            WK_CUDA(cudaEventRecord(g->t_ev[g->t_used + 1], g->stream));
-            g->t_used += 2;
+            r = bulk_event(g);
+            if (r) return r;
         }
         if (fork) {
             WK_CUDA(cudaEventRecord(g->ev_join, g->side));
@@ -841,6 +930,7 @@ int do_steps(wake_grid* g, int n) {
         for (int c = 0; c < 3; ++c) g->last_step_g[c] = g->phys.g[c];
         ++g->k;
     }
+    if (n > 0 && g->mem_on) wk::grid_force_left(g, by_rows);
     return WAKE_OK;
 }
 
@@ -849,9 +939,28 @@ int do_steps(wake_grid* g, int n) {
 namespace wk {
 
 bool grid_valid(wake_grid* g) { return valid_grid(g); }
-int grid_prepare(wake_grid* g) { return prepare(g); }
+int grid_prepare(wake_grid* g) {
+    int r = prepare_state(g);
+    if (!r) r = ensure_cells(g);
+    if (!r) r = ensure_units(g, g->cells);
+    if (!r && g->mem_list == 2) r = flush_force(g);
+    return r;
+}
 
-StepArgs grid_step_args(const wake_grid* g) {
+// Whether a state buffer of that many bytes is read evict-first (read_policy): up to three quarters of the L2, above
+// which it no longer helps (D3Q19 107 MB, 131 MB) and a batch of 108 MB lost 3 %.
+bool fits_l2(long long bytes) {
+    static int l2 = 0;
+    if (l2 == 0) {
+        int dev = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev) != cudaSuccess)
+            l2 = 126 << 20;
+    }
+    return bytes <= l2 / 4 * 3ll;
+}
+
+StepArgs grid_step_args(const wake_grid* g, bool rest) {
+    const CellList& L = rest ? g->rest : g->cells;
     StepArgs a{};
     a.flags = g->d_flags.as<uint8_t>();
     a.status = g->d_status.as<unsigned>();
@@ -860,23 +969,58 @@ StepArgs grid_step_args(const wake_grid* g) {
     a.mem.enabled = g->mem_on;
     if (g->mem_on) {
         for (int c = 0; c < 3; ++c) a.mem.center[c] = g->center[c];
-        a.mem.r_max = g->rmax;
-        a.mem.r_max_sq = g->rmax * g->rmax;
-        a.mem.warp_base = g->d_warp_base.as<int>();
-        a.mem.warps_per_row = g->warps_per_row;
-        a.mem.contrib = g->d_contrib.as<double>();
-        a.mem.n_nodes = g->n_mem_nodes;
+        a.mem.slot = L.slot.as<int>();
+        a.mem.slots = L.slots;
+        a.mem.contrib = L.contrib.as<double>();
+        a.mem.stride = L.stride;
+        a.mem.pending = g->d_counters.as<unsigned>();
         a.mem.hist_step = g->d_counters.as<unsigned>() + 1;
         a.mem.hist = g->d_hist.as<double>();
         a.mem.hist_cap = g->hist_cap;
     }
     a.phys = g->phys;
+    a.evict_first = fits_l2(static_cast<long long>(g->elem) * g->Q * g->pitch);
+    a.nodes = static_cast<unsigned>(g->N);
+    a.cells = rest ? 0u : static_cast<unsigned>((g->N + CELL - 1) / CELL);
+    a.cell_kind = g->d_kind.as<uint8_t>();
+    a.nunits = static_cast<unsigned>(L.units.size());
+    a.units = L.d_units.as<unsigned>();
+    a.list = L.list.as<uint4>();
+    a.records = L.records.as<uint4>();
+    a.row_kind = g->d_row_kind.as<uint8_t>();
     a.th = g->th;
     return a;
 }
 
+void grid_step_buffers(wake_grid* g, int cur, StepArgs& a) {
+    a.cur = a.reverse = cur;
+    a.fin = g->buf(cur);
+    a.fout = g->buf(1 - cur);
+    a.th.tin = g->tbuf(cur);
+    a.th.tout = g->tbuf(1 - cur);
+    const char* in = static_cast<const char*>(a.fin);
+    char* out = static_cast<char*>(a.fout);
+    const long long e = static_cast<long long>(g->elem);
+    for (int q = 0; q < g->Q; ++q) {
+        const long long plane = q * g->pitch * e;
+        const long long shift = g->lat.cx[q] + static_cast<long long>(g->nx) * (g->lat.cy[q] + static_cast<long long>(g->ny) * g->lat.cz[q]);
+        a.in[q] = in + plane;
+        a.pull[q] = in + plane - shift * e;
+        a.out[q] = out + plane;
+    }
+}
+
+void grid_force_left(wake_grid* g, bool rest) {
+    g->mem_list = rest ? 2 : 1;
+    g->mem_left = true;
+    ++g->mem_issued;
+    cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(g->stream, &s) == cudaSuccess && s != cudaStreamCaptureStatusNone) g->mem_captured = true;
+}
+
 void grid_advanced(wake_grid* g, int n) {
     if (n <= 0) return;
+    if (g->mem_on) grid_force_left(g, false);
     g->cur ^= (n & 1);
     g->k += n;
     g->mf_valid = false;
@@ -1422,9 +1566,12 @@ int wake_grid_enable_forces(wake_grid* g, float cx, float cy, float cz, float r_
     g->center[2] = (g->D == 3) ? cz : 0.f;
     g->rmax = r_max;
     g->hist_cap = history_capacity;
+    g->hist_seen = 0;
+    g->seen_at = ~0ull;
     WK_CUDA(g->d_hist.ensure(sizeof(double) * 3 * history_capacity));
     WK_CUDA(g->d_counters.ensure(sizeof(unsigned) * 2));
     WK_CUDA(cudaMemsetAsync(g->d_counters.p, 0, sizeof(unsigned) * 2, g->stream));
+    g->mem_list = 0;
     WK_CUDA(cudaMemsetAsync(g->d_hist.p, 0, sizeof(double) * 3 * history_capacity, g->stream));
     // the flags carry the momentum-exchange bit; a pending geometry change
     // is applied (with its state resync) by the next step instead
@@ -1453,14 +1600,20 @@ long long wake_grid_force_count(wake_grid* g) {
     if (cudaMemcpyAsync(c, g->d_counters.p, sizeof(c), cudaMemcpyDeviceToHost, g->stream) != cudaSuccess ||
         cudaStreamSynchronize(g->stream) != cudaSuccess)
         return set_error(WAKE_ERR_CUDA, "wake_grid_force_count: copy failed");
-    return c[1];
+    g->hist_seen = static_cast<long long>(c[1]) + (c[0] != 0u ? 1 : 0);  // with the outstanding one
+    g->seen_at = g->mem_issued;
+    return g->hist_seen;
 }
 
 int wake_grid_get_force_history(wake_grid* g, double* out, int max) {
     if (!valid_grid(g) || !out || max < 0) return set_error(WAKE_ERR_INVALID, "bad arguments");
     if (!g->mem_on) return 0;
-    const long long count = wake_grid_force_count(g);
+    // a caller asks for the count to size its buffer: no second wait for it unless steps came after
+    const bool seen = g->seen_at == g->mem_issued && !g->mem_captured;
+    const long long count = seen ? g->hist_seen : wake_grid_force_count(g);
     if (count < 0) return static_cast<int>(count);
+    const int r = flush_force(g);
+    if (r) return r;
     // the oldest step still in the ring, then at most `max` steps in order: one or two
     // contiguous runs of the ring, copied straight into the caller's buffer
     const long long cap = g->hist_cap;
@@ -1497,12 +1650,17 @@ static int capture_graph(wake_grid* g) {
     g->graph_ok = false;
     const int cur0 = g->cur;
     const long long k0 = g->k;
+    const int list0 = g->mem_list;
+    const bool left0 = g->mem_left, captured0 = g->mem_captured;
     cudaGraph_t graph = nullptr;
     WK_CUDA(cudaStreamBeginCapture(g->stream, cudaStreamCaptureModeThreadLocal));
     const int r = do_steps(g, g->graph_steps);
     cudaError_t e = cudaStreamEndCapture(g->stream, &graph);
     g->cur = cur0;
     g->k = k0;
+    g->mem_list = list0;
+    g->mem_left = left0;
+    g->mem_captured = captured0;
     if (r) {
         if (graph) cudaGraphDestroy(graph);
         return r;
@@ -1535,6 +1693,7 @@ int wake_grid_step(wake_grid* g, int n, float gx, float gy, float gz) {
             g->k += gs;
             g->mf_valid = false;
             for (int c = 0; c < 3; ++c) g->last_step_g[c] = g->phys.g[c];
+            if (g->mem_on) wk::grid_force_left(g, g->by_rows());
             done += gs;
         }
     }
@@ -1759,11 +1918,10 @@ int wake_grid_info(wake_grid* g, int* q, int* nx, int* ny, int* nz, int* storage
 long long wake_grid_device_bytes(wake_grid* g) {
     if (!valid_grid(g)) return WAKE_ERR_INVALID;
     const DevMem* all[] = {&g->A, &g->B, &g->d_types, &g->d_flags, &g->d_status, &g->d_nodestart, &g->d_link_node,
-                           &g->d_link_q, &g->d_link_delta, &g->d_link_mom, &g->d_counters, &g->d_hist,
-                           &g->d_warp_base, &g->d_contrib, &g->d_fast_rows, &g->d_gen_rows, &g->m_f, &g->m_rho,
-                           &g->m_ux, &g->m_uy, &g->m_uz, &g->m_speed, &g->m_diag, &g->TA, &g->TB, &g->m_t,
-                           &g->d_tiles, &g->d_gen4, &g->d_mixed, &g->m_an};
-    long long sum = 0;
+                           &g->d_link_rec, &g->d_link_mom, &g->d_counters, &g->d_hist, &g->d_kind, &g->d_seg, &g->d_row_kind,
+                           &g->d_row_list, &g->d_tiles, &g->m_f, &g->m_rho, &g->m_ux, &g->m_uy, &g->m_uz, &g->m_speed,
+                           &g->m_diag, &g->TA, &g->TB, &g->m_t, &g->m_an};
+    long long sum = static_cast<long long>(g->cells.bytes() + g->rest.bytes());
     for (const DevMem* m : all) sum += static_cast<long long>(m->bytes);
     return sum;
 }
@@ -1818,7 +1976,7 @@ int wake_grid_set_block(wake_grid* g, int threads_per_block) {
     if (threads_per_block < 32 || threads_per_block > 512 || threads_per_block % 32)
         return set_error(WAKE_ERR_INVALID, "threads per block must be a multiple of 32 in [32, 512]");
     g->choose_block(threads_per_block);
-    g->geom_dirty = true;  // momentum-exchange block slots depend on the launch shape
+    g->invalidate_graph();
     return WAKE_OK;
 }
 
@@ -1843,9 +2001,7 @@ int wake_grid_launches_per_step(wake_grid* g) {
     if (!valid_grid(g)) return WAKE_ERR_INVALID;
     const int r = prepare(g);
     if (r) return r;
-    if (g->use_tiles()) return 1 + (g->mem_on ? 1 : 0);
-    if (g->use_pipe() || g->use_rows()) return 1 + (g->n_mixed > 0 ? 1 : 0) + (g->n_gen > 0 ? 1 : 0) + (g->mem_on ? 1 : 0);
-    return (g->n_fast > 0 ? 1 : 0) + (g->n_gen > 0 ? 1 : 0) + (g->mem_on ? 1 : 0);
+    return g->by_rows() ? (g->n_row_fast > 0 ? 1 : 0) + (!g->rest.units.empty() || g->mem_on ? 1 : 0) : 1;
 }
 
 int wake_grid_time_bulk_launches(wake_grid* g, int on) {
@@ -1867,8 +2023,7 @@ int wake_grid_bulk_launch_times(wake_grid* g, double* total_ms, long long* launc
     }
     if (total_ms) *total_ms = sum;
     if (launches) *launches = static_cast<long long>(g->t_used / 2);
-    // the persistent launch also updates the general rows
-    if (nodes_per_launch) *nodes_per_launch = g->use_tiles() ? g->N : (g->use_pipe() || g->use_rows() ? g->row_fast_nodes : g->fast_nodes());
+    if (nodes_per_launch) *nodes_per_launch = g->by_rows() ? static_cast<long long>(g->n_row_fast) * g->nx : g->cell_nodes;
     g->t_used = 0;
     return WAKE_OK;
 }

@@ -45,14 +45,29 @@ struct RasterShape {
     float p[4];   // circle / sphere: r^2; ellipse: cos, sin, 1/a^2, 1/b^2
 };
 
-cudaError_t launch_step_any(int Q, int coll, int store, bool les, const StepArgs& a, const Launch& L, bool fast);
-cudaError_t launch_batch_any(int Q, int coll, int store, bool les, const BatchArgs& b, int tpb, cudaStream_t stream,
-                             bool fast, bool idx32);
+cudaError_t launch_cells_any(int Q, int coll, int store, bool les, const StepArgs& a, int tpb, cudaStream_t stream);
+cudaError_t launch_batch_any(int Q, int coll, int store, bool les, const BatchArgs& b, bool thermal, int tpb,
+                             cudaStream_t stream);
 cudaError_t launch_tiles_any(int Q, int coll, int store, bool les, const StepArgs& a, const TileArgs& t,
                              cudaStream_t stream);
 cudaError_t launch_rows_any(int Q, int store, bool les, const StepArgs& a, int rows, int tpb, cudaStream_t stream);
 cudaError_t launch_rows_pipe_any(int Q, int store, bool les, int cap, const StepArgs& a, const PipeArgs& p,
                                  cudaStream_t stream);
+
+// Listed cells of k_step_cells on the device (cells.cuh), for one set of flags.
+struct CellList {
+    DevMem list, records, d_units, slot, contrib;
+    unsigned general = 0;               // the first cells of `list`, with records; the others are pure
+    std::vector<uint4> cells;           // the list with its LIST_* bits
+    std::vector<unsigned> units;        // for `mode` (0: not made yet)
+    int mode = 0, slots = 0;
+    long long stride = 3;               // doubles of one half of contrib
+    unsigned long long version = 0;     // geom_version it was built for (0: never)
+    void release() {
+        for (DevMem* m : {&list, &records, &d_units, &slot, &contrib}) m->release();
+    }
+    std::size_t bytes() const { return list.bytes + records.bytes + d_units.bytes + slot.bytes + contrib.bytes; }
+};
 
 }  // namespace wk
 
@@ -97,70 +112,62 @@ struct wake_grid {
 
     std::vector<int> link_node, link_q;
     std::vector<float> link_delta, link_uw;  // uw: 3 per link
-    DevMem d_link_node, d_link_q, d_link_delta, d_link_mom;
+    DevMem d_link_node, d_link_rec, d_link_mom;
+    std::vector<int> dev_link_node;  // node of each uploaded link
     int dev_links = 0;         // links currently on the device (the flags refer to these)
     bool links_dirty = false;  // host links differ from the device copy
 
     int mem_on = 0, hist_cap = 0;
     float center[3] = {0.f, 0.f, 0.f}, rmax = 0.f;
-    DevMem d_counters, d_hist;         // counters: [0] unused, [1] history entries written
-    DevMem d_warp_base, d_contrib;     // momentum-exchange slots (see MemCfg)
-    int warps_per_row = 1, n_mem_nodes = 0;
+    DevMem d_counters, d_hist;  // counters: [0] outstanding force (MemCfg::pending), [1] history entries written
+    // the history's length as read last, the value of mem_issued then (~0: never); calls that issued steps with forces on
+    long long hist_seen = 0;
+    unsigned long long seen_at = ~0ull, mem_issued = 0;
+    // whose slots the last step left its force in (0 none, 1 `cells`, 2 `rest`), whether it may still be outstanding, and
+    // whether steps were captured into a caller's graph, whose replays leave forces unseen by the host
+    int mem_list = 0;
+    bool mem_left = false, mem_captured = false;
 
-    // pure-gather spans (0, row, x0, x1) handled by k_step_fast, and general segments
-    // (SEG nodes of a row, numbered row * nseg + s) handled by k_step
-    DevMem d_fast_rows, d_gen_rows;
-    int n_fast = 0, n_gen = 0;
-    std::vector<uint4> h_fast_rows;     // spans
-    std::vector<unsigned> h_gen_rows;   // general segments
-    long long fast_nodes() const {      // nodes in the pure-gather spans
-        long long n = 0;
-        for (const uint4& sp : h_fast_rows) n += sp.w - sp.z;
-        return n;
-    }
+    // k_step_cells: what the linear cells and the segments are, and the cells that are listed
+    DevMem d_kind, d_seg;
+    unsigned long long seg_version = 0;  // geom_version of d_seg
+    std::vector<uint8_t> h_kind, h_seg;
+    wk::CellList cells;
+    unsigned long long units_version = 0;  // a fresh number whenever units are made (next_geom_version)
+    long long cell_nodes = 0;  // nodes of the segments that are not all solid
     // Identity of the current flags / row lists: a fresh process-wide number at every
     // rebuild (next_geom_version), so a batch never takes a new grid that happens to
     // reuse a destroyed grid's address for the old one.
     unsigned long long geom_version = 0;
 
-    int tpb = 0, xchunks = 1, rows = 1, tpb_fast = 64;
-    // step kernels: 0 automatic, 1 direct (k_step_fast for the pure-gather rows beside
-    // k_step for the rest), 2 persistent tiles (k_step_tiles: pure-gather tiles staged in
-    // shared memory plus the general rows, when the row shape allows it)
+    int tpb = 0, xchunks = 1, rows = 1, tpb_cells = 64;
+    // step kernels: 0 automatic, 1 direct (k_step_cells over the whole lattice), 2 to 4 a bulk kernel for the
+    // rows whose every node is a pure gather (ROW_FAST) beside k_step_cells for the other rows (`rest`):
+    // 2 persistent tiles (k_step_tiles), 3 one block per row (k_step_rows, TRT), 4 rows moved through shared
+    // memory by bulk copies (k_step_rows_pipe, TRT; the automatic choice for 16-bit storage).
     int kernel_variant = 0;
-    bool use_tiles() const { return kernel_variant == 2 && wk::tile_row_ok(nx, static_cast<int>(elem)); }
-    // Whole-row TRT kernel (k_step_rows, variant 3): one block per row over the rows whose
-    // every node is a pure gather (d_row_kind, ROW_* bytes); the pure-gather runs of the other
-    // rows (d_mixed) go to k_step_fast beside the general segments. Not automatic: on the D3Q19
-    // sphere channel the span kernel moves FP32 rows 3 % faster per node.
-    DevMem d_row_kind;
-    int n_row_fast = 0;           // rows marked ROW_FAST
-    long long row_fast_nodes = 0;  // nodes in them
-    bool use_rows() const {
-        return kernel_variant == 3 && collision == WAKE_TRT && nx % 2 == 0 &&
-               static_cast<long long>(Q) * pitch < (1ll << 32) && !th.on && n_row_fast > 0;
-    }
-    int tpb_rows() const { return nx <= 64 ? 32 : 64; }
-    // Pipelined whole-row kernel (k_step_rows_pipe, variant 4, and the automatic choice for
-    // 16-bit storage): the ROW_FAST rows as (row | descriptor << 28), staged through shared
-    // memory by bulk copies. FP32 takes the span kernel automatically (measured faster there:
-    // three CTAs per SM fill the shared memory).
-    DevMem d_row_list;
+    DevMem d_row_kind, d_row_list, d_tiles;  // ROW_* byte per row; ROW_FAST rows (row | bits << 28); tiles of them
+    int n_row_fast = 0, n_tiles = 0;
+    wk::CellList rest;
+    bool narrow() const { return static_cast<long long>(Q) * pitch < (1ll << 32); }
+    bool tiles_fit() const { return kernel_variant == 2 && wk::tile_row_ok(nx, static_cast<int>(elem)) && !th.on; }
+    bool rows_fit() const { return kernel_variant == 3 && collision == WAKE_TRT && nx % 2 == 0 && narrow() && !th.on; }
     int pipe_cap() const { return nx <= 256 ? 256 : 512; }
-    bool use_pipe() const {
+    bool pipe_fits() const {
         const bool chosen = kernel_variant == 4 || (kernel_variant == 0 && storage != 0);
         return chosen && collision == WAKE_TRT && nx % 2 == 0 && nx <= 512 &&
-               (static_cast<long long>(nx) * static_cast<long long>(elem)) % 16 == 0 &&
-               static_cast<long long>(Q) * pitch < (1ll << 32) && !th.on && n_row_fast > 0 && rows < (1 << 28);
+               (static_cast<long long>(nx) * static_cast<long long>(elem)) % 16 == 0 && narrow() && !th.on &&
+               rows < (1 << 28);
     }
-    // pure-gather tiles (0, (z << 16) | y0, rows, 0) and the segments of the other rows
-    // (0, segment, general-segment entry, 0)
-    DevMem d_tiles, d_gen4, d_mixed;
-    int n_tiles = 0, n_tile_gen = 0, n_mixed = 0;
-    std::vector<uint4> h_tiles, h_gen4, h_mixed;  // h_mixed: the spans of rows outside the tiles
+    // (the row tables of the current flags exist once prepared)
+    bool use_tiles() const { return tiles_fit(); }
+    bool use_rows() const { return rows_fit() && n_row_fast > 0; }
+    bool use_pipe() const { return pipe_fits() && n_row_fast > 0; }
+    bool by_rows() const { return use_tiles() || use_rows() || use_pipe(); }
+    int tpb_rows() const { return nx <= 64 ? 32 : 64; }
     cudaStream_t stream = nullptr;
     bool own_stream = false;
-    cudaStream_t side = nullptr;  // forked stream of the general-row launch
+    cudaStream_t side = nullptr;  // forked stream of the rows beside a bulk kernel
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     long long k = 0;
 
@@ -193,10 +200,11 @@ struct wake_grid {
         if (stream) idle = cudaStreamSynchronize(stream) == cudaSuccess;
         if (side) idle = idle && cudaStreamSynchronize(side) == cudaSuccess;
         if (idle) {
-            DevMem* all[] = {&A, &B, &d_types, &d_flags, &d_status, &d_nodestart, &d_link_node, &d_link_q,
-                             &d_link_delta, &d_link_mom, &d_counters, &d_hist, &d_warp_base, &d_contrib,
-                             &d_fast_rows, &d_gen_rows, &d_tiles, &d_gen4, &d_mixed, &d_row_kind, &d_row_list, &m_f, &m_rho, &m_ux, &m_uy, &m_uz,
-                             &m_speed, &m_diag, &TA, &TB, &m_t, &m_an};
+            DevMem* all[] = {&A, &B, &d_types, &d_flags, &d_status, &d_nodestart, &d_link_node, &d_link_rec,
+                             &d_link_mom, &d_counters, &d_hist, &d_kind, &d_seg, &d_row_kind, &d_row_list, &d_tiles, &m_f,
+                             &m_rho, &m_ux, &m_uy, &m_uz, &m_speed, &m_diag, &TA, &TB, &m_t, &m_an};
+            cells.release();
+            rest.release();
             for (DevMem* m : all) m->release();
         }
         for (cudaEvent_t e : t_ev) cudaEventDestroy(e);
@@ -214,6 +222,8 @@ struct wake_grid {
         g.nx = nx;
         g.ny = ny;
         g.nz = nz;
+        g.by_nx = wk::FastDiv::of(static_cast<unsigned>(nx));
+        g.by_ny = wk::FastDiv::of(static_cast<unsigned>(ny));
         g.periodic_y = (D == 3) ? periodic_y : 0;
         g.periodic_z = (D == 3) ? periodic_z : 0;
         g.pitch = pitch;
@@ -229,14 +239,12 @@ struct wake_grid {
     Links links() const {
         Links l{};
         l.node_start = d_nodestart.as<int>();
-        l.node = d_link_node.as<int>();
-        l.q = d_link_q.as<int>();
-        l.delta = d_link_delta.as<float>();
+        l.rec = d_link_rec.as<uint4>();
         l.mom = d_link_mom.as<float>();
         l.count = dev_links;
         return l;
     }
-    Launch launch() const { return Launch{tpb, xchunks, rows, stream, ny, nz, tpb_fast}; }
+    Launch launch() const { return Launch{tpb, xchunks, rows, stream, ny, nz, tpb_cells}; }
     int blocks() const { return rows * xchunks; }
 
     void invalidate_graph() { graph_ok = false; }
@@ -260,19 +268,7 @@ struct wake_grid {
         }
         xchunks = (nx + tpb - 1) / tpb;
         rows = ny * nz;
-        // k_step_fast is limited to WK_FAST_MAX_THREADS threads. Least idle lanes over the row,
-        // ties to the smaller block: 64-thread blocks measured fastest on 256-node rows (more
-        // independent blocks in flight per SM, shorter tail per row).
-        const int cap = std::min(want > 0 ? want : WK_FAST_MAX_THREADS, WK_FAST_MAX_THREADS);
-        int best = -1, best_waste = 1 << 30;
-        for (int t = 64; t <= cap; t += 32) {
-            const int waste = ((nx + t - 1) / t) * t - nx;
-            if (waste < best_waste) {
-                best = t;
-                best_waste = waste;
-            }
-        }
-        tpb_fast = best > 0 ? best : 64;
+        tpb_cells = want > 0 ? std::max(32, std::min(want, WK_FAST_MAX_THREADS)) : WK_FAST_MAX_THREADS;
     }
 };
 
@@ -281,11 +277,18 @@ namespace wk {
 // Validity check that records the error (WAKE_ERR_INVALID) for a null handle.
 bool grid_valid(wake_grid* g);
 // Bring a lattice to the point where its state buffers hold Collide(f^k) for the
-// current geometry and parameters (rebuilds flags, re-collides when pending).
+// current geometry and parameters (rebuilds flags, re-collides when pending) and
+// its cell list is built.
 int grid_prepare(wake_grid* g);
 unsigned long long next_geom_version();
-// Step arguments of one lattice (rows and buffers left for the caller).
-StepArgs grid_step_args(const wake_grid* g);
+// Step arguments of one lattice: the direct range and its listed cells, or the rows beside a bulk kernel
+// (buffers left for the caller).
+StepArgs grid_step_args(const wake_grid* g, bool rest = false);
+bool fits_l2(long long bytes);
+// Its buffers: the state in buf(cur), the step's output in the other one.
+void grid_step_buffers(wake_grid* g, int cur, StepArgs& a);
+// The last step left its force in the slots of `rest` (else `cells`).
+void grid_force_left(wake_grid* g, bool rest);
 // Bookkeeping after n steps run outside wake_grid_step (by a batch).
 void grid_advanced(wake_grid* g, int n);
 // Error status word of the lattice: WAKE_OK or WAKE_ERR_NUMERIC (synchronizes its stream).

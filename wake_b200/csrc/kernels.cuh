@@ -4,6 +4,7 @@
 
 #include <cuda_runtime.h>
 
+#include "cells.cuh"
 #include "rowpipe.cuh"
 #include "rows.cuh"
 #include "staged.cuh"
@@ -17,7 +18,7 @@ struct Launch {
     int rows;      // ny * nz
     cudaStream_t stream;
     int ny, nz;
-    int tpb_fast;  // threads per block of k_step_fast (<= 256; one warp per segment)
+    int tpb_cells;  // threads per block of k_step_cells
 };
 
 struct FlagCfg {
@@ -30,9 +31,9 @@ struct FlagCfg {
 
 // Per-lattice entry points (defined once per Q in kernels_impl.cuh).
 #define WK_DECLARE_LAUNCHERS(Q)                                                                                   \
-    cudaError_t launch_step_q##Q(int coll, int store, bool les, const StepArgs& a, const Launch& L, bool fast);  \
-    cudaError_t launch_batch_q##Q(int coll, int store, bool les, const BatchArgs& b, int tpb,                   \
-                                  cudaStream_t stream, bool fast, bool idx32);                                  \
+    cudaError_t launch_cells_q##Q(int coll, int store, bool les, StepArgs a, int tpb, cudaStream_t stream);       \
+    cudaError_t launch_batch_q##Q(int coll, int store, bool les, BatchArgs b, bool thermal, int tpb,              \
+                                  cudaStream_t stream);                                                           \
     cudaError_t launch_tiles_q##Q(int coll, int store, bool les, const StepArgs& a, const TileArgs& t,          \
                                   cudaStream_t stream);                                                          \
     cudaError_t launch_materialise_q##Q(int store, const void* fin, const uint8_t* flags, const Geo& geo,        \
@@ -42,8 +43,8 @@ struct FlagCfg {
                                     const uint8_t* flags, const Geo& geo, const Physics& phys, const Launch& L); \
     cudaError_t launch_flags_q##Q(const uint8_t* types, uint8_t* flags, const Geo& geo, const FlagCfg& cfg,      \
                                   const Launch& L);                                                              \
-    cudaError_t launch_seg_class_q##Q(const uint8_t* flags, uint8_t* cls, const Geo& geo, long long nsegs,       \
-                                      cudaStream_t stream);                                                      \
+    cudaError_t launch_records_q##Q(const uint8_t* flags, uint4* list, unsigned n, unsigned general, uint4* records,   \
+                                    const Links& links, const Geo& geo, const FlagCfg& cfg, cudaStream_t stream);     \
     cudaError_t launch_rows_q##Q(int store, bool les, const StepArgs& a, int rows, int tpb, cudaStream_t stream); \
     cudaError_t launch_rows_pipe_q##Q(int store, bool les, int cap, const StepArgs& a, const PipeArgs& p,         \
                                       cudaStream_t stream);

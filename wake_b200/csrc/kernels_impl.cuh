@@ -76,27 +76,63 @@ __global__ void k_flags(const uint8_t* __restrict__ types, uint8_t* __restrict__
     flags[i] = fl;
 }
 
-// Segment classes for the two step kernels (one warp per segment of SEG nodes):
-// bit 0 = every node is a pure gather (k_step_fast), bit 1 = the segment holds
-// a momentum-exchange node, bit 2 = every node is solid (no launch needed).
+// Node records of the listed general cells (cells.cuh), one block of CELL threads per cell, and every listed cell's
+// LIST_* bits: the first `general` are general, the others pure.
 template <int Q>
-__global__ void k_seg_class(const uint8_t* __restrict__ flags, uint8_t* __restrict__ cls, const Geo geo,
-                            long long nsegs) {
-    const long long e = blockIdx.x * static_cast<long long>(blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (e >= nsegs) return;
-    const Seg sg = seg_decode(static_cast<unsigned>(e), geo);
-    const int lane = threadIdx.x & 31;
-    int fast = 1, mem = 0, solid = 1;
-    for (int x = sg.x0 + lane; x < sg.x1; x += 32) {
-        const uint8_t fl = flags[sg.row0 + x];
-        fast &= (fl & FL_FAST) ? 1 : 0;
-        mem |= (fl & FL_MEM) ? 1 : 0;
-        solid &= (fl & FL_TYPE) == CT_SOLID ? 1 : 0;
+__global__ void __launch_bounds__(CELL)
+    k_records(const uint8_t* __restrict__ flags, uint4* __restrict__ list, unsigned general,
+              uint4* __restrict__ records, const Links links, const Geo geo, const FlagCfg cfg) {
+    using L = Lat<Q>;
+    const uint4 c = list[blockIdx.x];
+    if (blockIdx.x >= general) {
+        const bool zh = threadIdx.x < c.y && (flags[c.x + threadIdx.x] & (FL_ZH_IN | FL_ZH_OUT));
+        if (__syncthreads_or(zh) && threadIdx.x == 0) list[blockIdx.x].y = c.y | LIST_ZH;
+        return;
     }
-    fast = __all_sync(0xffffffffu, fast);
-    mem = __any_sync(0xffffffffu, mem);
-    solid = __all_sync(0xffffffffu, solid);
-    if (lane == 0) cls[e] = static_cast<uint8_t>((fast ? 1 : 0) | (mem ? 2 : 0) | (solid ? 4 : 0));
+    uint4 r = make_uint4(0u, 0u, 0u, 0u);
+    if (threadIdx.x < c.y) {
+        const unsigned i = c.x + threadIdx.x;
+        const uint8_t fl = flags[i];
+        if ((fl & FL_TYPE) != CT_SOLID) {
+            r.x = CN_LIVE | (fl & FL_ZH_IN ? CN_ZH_IN : 0u) | (fl & FL_ZH_OUT ? CN_ZH_OUT : 0u);
+            unsigned hit = 0;
+            if (fl & FL_BFL) {
+                const int first = links.node_start[i];
+                r.w = (static_cast<unsigned>(first) - c.z) << CN_LINK_SHIFT;
+                for (int k = first; k < links.count && links.rec[k].x == i; ++k) r.w |= 1u << ((links.rec[k].z >> 16) & 0xffu);
+            }
+            const int row = static_cast<int>(i / geo.nx), x = static_cast<int>(i % geo.nx);
+            const int y = row % geo.ny, z = row / geo.ny;
+#pragma unroll
+            for (int q = 1; q < Q; ++q) {
+                const int sx = L::cx(q) ? wrap<Q>(x - L::cx(q), geo.nx) : x;
+                int sy = y - L::cy(q), sz = z - L::cz(q);
+                if (L::cy(q) && geo.periodic_y) sy = wrap<Q>(sy, geo.ny);
+                if (L::cz(q) && geo.periodic_z) sz = wrap<Q>(sz, geo.nz);
+                if (sy < 0 || sy >= geo.ny || sz < 0 || sz >= geo.nz) {
+                    r.x |= 1u << q;  // half-way wall at the lattice's face
+                    if (Q == 9) r.z |= 1u << (CN_WALL_SHIFT + q);
+                    continue;
+                }
+                const uint8_t t = flags[(static_cast<long long>(sz) * geo.ny + sy) * geo.nx + sx] & FL_TYPE;
+                if (t == CT_SOLID || t == CT_MOVING_WALL) {
+                    r.x |= 1u << q;
+                    hit |= 1u << q;
+                    if (t == CT_MOVING_WALL) r.z |= 1u << q;
+                }
+            }
+            if (fl & FL_MEM) r.y = mem_links<Q>(hit, x, y, z, geo, cfg.center, cfg.r_max, cfg.r_max_sq);
+        }
+    }
+    records[static_cast<long long>(blockIdx.x) * CELL + threadIdx.x] = r;
+    const bool live = (r.x & CN_LIVE) != 0u;
+    const unsigned half = threadIdx.x >> 5;
+    unsigned bits = 0;
+    for (unsigned h = 0; h < 2; ++h) {
+        if (__syncthreads_or(half == h && live)) bits |= LIST_LIVE << h;
+        if (__syncthreads_or(half == h && r.y != 0u)) bits |= LIST_MEM << h;
+    }
+    if (threadIdx.x == 0) list[blockIdx.x].y = c.y | bits;
 }
 
 // Pull-free read of f^0 (state buffer holding pre-collision populations).
@@ -139,34 +175,40 @@ __global__ void __launch_bounds__(512) k_direct(const void* fin_v, const uint8_t
 namespace {
 constexpr int kQ = WK_Q;
 
-template <int C, int S, bool LES>
-void step_one(const StepArgs& a, const Launch& L, bool fast) {
-    if (fast) {
-        if (a.nspans <= 0) return;
-        // one block per span; 32-bit element indexing whenever every index of the state buffer fits
-        const bool idx32 = static_cast<long long>(kQ) * a.geo.pitch < (1ll << 32);
-        if (idx32) k_step_fast<kQ, C, S, LES, true><<<a.nspans, L.tpb_fast, 0, L.stream>>>(a);
-        else k_step_fast<kQ, C, S, LES, false><<<a.nspans, L.tpb_fast, 0, L.stream>>>(a);
-    } else {
-        if (a.nrows <= 0) return;
-        k_step<kQ, C, S, LES><<<a.nrows, SEG, 0, L.stream>>>(a);
-    }
+unsigned blocks_of(unsigned units, int tpb) {
+    const unsigned wpb = static_cast<unsigned>(tpb) / 32u;
+    return (units + wpb - 1u) / wpb;
+}
+
+// Blocks of a launch over `units` pure units, and how they are laid out. Two units per warp where the blocks
+// still fill the device (148 SMs, 10 or more blocks each) several times over: a block's start costs about a tenth
+// of a one-unit block's life (D3Q19 FP32 160^3: 110.5 us with one, 106.6 with two, 113 with eight); smaller
+// lattices need the blocks to even out the end (97^3: 27.3 / 26.8 / 29.8).
+unsigned plan(unsigned units, int tpb, unsigned list_blocks, unsigned& run, unsigned& spread) {
+    unsigned blocks = blocks_of(units, tpb);
+    run = blocks >= 148u * 64u ? 2u : 1u;
+    blocks = list_blocks + (blocks + run - 1u) / run;
+    spread = 0;
+    while (list_blocks && (static_cast<unsigned long long>(list_blocks) << (spread + 1)) <= blocks / 5ull * 3ull) ++spread;
+    return blocks;
+}
+
+template <int C, int S, bool LES, bool TH>
+void cells_one(StepArgs& a, int tpb, cudaStream_t st) {
+    a.list_blocks = blocks_of(a.nunits + (a.mem.enabled ? 1u : 0u), tpb);
+    const unsigned blocks = plan(a.cells * pure_units<kQ, C, S, TH>(), tpb, a.list_blocks, a.run, a.spread);
+    if (blocks) k_step_cells<kQ, C, S, LES, TH><<<blocks, tpb, 0, st>>>(a);
+}
+template <int C, int S, bool LES, bool TH>
+void batch_one(BatchArgs& b, int tpb, cudaStream_t st) {
+    b.list_blocks = blocks_of(b.nlisted, tpb);
+    const unsigned blocks = plan(b.npure * pure_units<kQ, C, S, false>(), tpb, b.list_blocks, b.run, b.spread);
+    if (blocks) k_step_cells_batch<kQ, C, S, LES, TH><<<blocks, tpb, 0, st>>>(b);
 }
 template <int C, int S, bool LES>
 void initial_one(const float* f0, void* A, void* B, const uint8_t* flags, const Geo& g, const Physics& p,
                  const Launch& L) {
     k_initial<kQ, C, S, LES><<<L.rows * L.xchunks, L.tpb, 0, L.stream>>>(f0, A, B, flags, g, p, L.xchunks);
-}
-template <int C, int S, bool LES>
-void batch_one(const BatchArgs& b, int tpb, cudaStream_t st, bool fast, bool idx32) {
-    if (fast) {
-        if (b.nspans <= 0) return;
-        if (idx32) k_step_fast_batch<kQ, C, S, LES, true><<<b.nspans, tpb, 0, st>>>(b);
-        else k_step_fast_batch<kQ, C, S, LES, false><<<b.nspans, tpb, 0, st>>>(b);
-    } else {
-        if (b.nrows <= 0) return;
-        k_step_batch<kQ, C, S, LES><<<b.nrows, SEG, 0, st>>>(b);
-    }
 }
 // Persistent tile kernel: TILE_CTAS_PER_SM CTAs per SM (capped by the work), dynamic shared
 // memory opted in once per kernel instantiation.
@@ -190,51 +232,55 @@ cudaError_t tiles_launch(unsigned smem, int work, cudaStream_t st, const StepArg
 template <int C, int S, bool LES>
 cudaError_t tiles_one(const StepArgs& a, const TileArgs& t, cudaStream_t st) {
     constexpr unsigned smem = tile_smem_bytes<kQ, S>();
-    const int work = std::max(std::max(t.ntiles, t.ngen), t.nspans);
-    if (work <= 0) return cudaSuccess;
-    if (t.dom) return tiles_launch<k_step_tiles<kQ, C, S, LES, true>>(smem, work, st, a, t);
-    return tiles_launch<k_step_tiles<kQ, C, S, LES, false>>(smem, work, st, a, t);
+    if (t.ntiles <= 0) return cudaSuccess;
+    return tiles_launch<k_step_tiles<kQ, C, S, LES>>(smem, t.ntiles, st, a, t);
 }
 using TilesFn = cudaError_t (*)(const StepArgs&, const TileArgs&, cudaStream_t);
-using StepFn = void (*)(const StepArgs&, const Launch&, bool);
-using BatchFn = void (*)(const BatchArgs&, int, cudaStream_t, bool, bool);
+using CellsFn = void (*)(StepArgs&, int, cudaStream_t);
+using BatchFn = void (*)(BatchArgs&, int, cudaStream_t);
 using InitFn = void (*)(const float*, void*, void*, const uint8_t*, const Geo&, const Physics&, const Launch&);
 
-#define WK_ROW(C, S) {step_one<C, S, false>, step_one<C, S, true>}
+#if WK_Q == 9  // [LES][coupled temperature]
+#define WK_4(F, C, S) {{F<C, S, false, false>, F<C, S, false, true>}, {F<C, S, true, false>, F<C, S, true, true>}}
+#else
+#define WK_4(F, C, S) {{F<C, S, false, false>, nullptr}, {F<C, S, true, false>, nullptr}}
+#endif
+#define WK_TABLE(F)                                                                    \
+    {{WK_4(F, 0, 0), WK_4(F, 0, 1), WK_4(F, 0, 2), WK_4(F, 0, 3)},                     \
+     {WK_4(F, 1, 0), WK_4(F, 1, 1), WK_4(F, 1, 2), WK_4(F, 1, 3)},                     \
+     {WK_4(F, 2, 0), WK_4(F, 2, 1), WK_4(F, 2, 2), WK_4(F, 2, 3)}}
+const CellsFn kCells[3][4][2][2] = WK_TABLE(cells_one);
+const BatchFn kBatch[3][4][2][2] = WK_TABLE(batch_one);
+#undef WK_4
+#undef WK_TABLE
 #define WK_IROW(C, S) {initial_one<C, S, false>, initial_one<C, S, true>}
-const StepFn kStep[3][4][2] = {{WK_ROW(0, 0), WK_ROW(0, 1), WK_ROW(0, 2), WK_ROW(0, 3)},
-                               {WK_ROW(1, 0), WK_ROW(1, 1), WK_ROW(1, 2), WK_ROW(1, 3)},
-                               {WK_ROW(2, 0), WK_ROW(2, 1), WK_ROW(2, 2), WK_ROW(2, 3)}};
 const InitFn kInit[3][4][2] = {{WK_IROW(0, 0), WK_IROW(0, 1), WK_IROW(0, 2), WK_IROW(0, 3)},
                                {WK_IROW(1, 0), WK_IROW(1, 1), WK_IROW(1, 2), WK_IROW(1, 3)},
                                {WK_IROW(2, 0), WK_IROW(2, 1), WK_IROW(2, 2), WK_IROW(2, 3)}};
-#define WK_BROW(C, S) {batch_one<C, S, false>, batch_one<C, S, true>}
-const BatchFn kBatch[3][4][2] = {{WK_BROW(0, 0), WK_BROW(0, 1), WK_BROW(0, 2), WK_BROW(0, 3)},
-                                 {WK_BROW(1, 0), WK_BROW(1, 1), WK_BROW(1, 2), WK_BROW(1, 3)},
-                                 {WK_BROW(2, 0), WK_BROW(2, 1), WK_BROW(2, 2), WK_BROW(2, 3)}};
 #define WK_SROW(C, S) {tiles_one<C, S, false>, tiles_one<C, S, true>}
 const TilesFn kTiles[3][4][2] = {{WK_SROW(0, 0), WK_SROW(0, 1), WK_SROW(0, 2), WK_SROW(0, 3)},
                                  {WK_SROW(1, 0), WK_SROW(1, 1), WK_SROW(1, 2), WK_SROW(1, 3)},
                                  {WK_SROW(2, 0), WK_SROW(2, 1), WK_SROW(2, 2), WK_SROW(2, 3)}};
-#undef WK_ROW
 #undef WK_IROW
-#undef WK_BROW
 #undef WK_SROW
 
 bool valid(int coll, int store) { return coll >= 0 && coll < 3 && store >= 0 && store < 4; }
 }  // namespace
 
-cudaError_t WK_CAT(launch_step_q, WK_Q)(int coll, int store, bool les, const StepArgs& a, const Launch& L,
-                                       bool fast) {
+cudaError_t WK_CAT(launch_cells_q, WK_Q)(int coll, int store, bool les, StepArgs a, int tpb, cudaStream_t stream) {
     if (!valid(coll, store)) return cudaErrorInvalidValue;
-    kStep[coll][store][les ? 1 : 0](a, L, fast);
+    const CellsFn f = kCells[coll][store][les ? 1 : 0][a.th.on ? 1 : 0];
+    if (!f) return cudaErrorInvalidValue;
+    f(a, tpb, stream);
     return cudaGetLastError();
 }
 
-cudaError_t WK_CAT(launch_batch_q, WK_Q)(int coll, int store, bool les, const BatchArgs& b, int tpb,
-                                        cudaStream_t stream, bool fast, bool idx32) {
+cudaError_t WK_CAT(launch_batch_q, WK_Q)(int coll, int store, bool les, BatchArgs b, bool thermal, int tpb,
+                                        cudaStream_t stream) {
     if (!valid(coll, store)) return cudaErrorInvalidValue;
-    kBatch[coll][store][les ? 1 : 0](b, tpb, stream, fast, idx32);
+    const BatchFn f = kBatch[coll][store][les ? 1 : 0][thermal ? 1 : 0];
+    if (!f) return cudaErrorInvalidValue;
+    f(b, tpb, stream);
     return cudaGetLastError();
 }
 
@@ -388,11 +434,11 @@ cudaError_t WK_CAT(launch_rows_pipe_q, WK_Q)(int store, bool les, int cap, const
     }
 }
 
-cudaError_t WK_CAT(launch_seg_class_q, WK_Q)(const uint8_t* flags, uint8_t* cls, const Geo& geo, long long nsegs,
-                                            cudaStream_t stream) {
-    if (nsegs <= 0) return cudaSuccess;
-    const long long blocks = (nsegs + 7) / 8;
-    k_seg_class<kQ><<<static_cast<unsigned>(blocks), 256, 0, stream>>>(flags, cls, geo, nsegs);
+cudaError_t WK_CAT(launch_records_q, WK_Q)(const uint8_t* flags, uint4* list, unsigned n, unsigned general,
+                                          uint4* records, const Links& links, const Geo& geo, const FlagCfg& cfg,
+                                          cudaStream_t stream) {
+    if (n == 0) return cudaSuccess;
+    k_records<kQ><<<n, CELL, 0, stream>>>(flags, list, general, records, links, geo, cfg);
     return cudaGetLastError();
 }
 

@@ -31,7 +31,7 @@
 // of 16 bytes (bulk copies move whole 16-byte units from 16-byte-aligned
 // addresses; the plane pitch is a multiple of 64 elements); Q * pitch < 2^32; no
 // coupled temperature. The per-node arithmetic is trt_pairs2's, so results equal
-// the span and row kernels' bit for bit.
+// the cell and row kernels' bit for bit.
 #pragma once
 
 #include "rows.cuh"
@@ -97,7 +97,7 @@ __device__ __forceinline__ void pull_shift(int q, int& cy, int& cz) {
 // Producer lane q (< Q) copies direction q's source row of `row` into its slot of the stage
 // (shared address `stage`); lane 0 posts the byte count first. All lanes issue at once.
 template <int Q, int CAP, class T>
-__device__ __forceinline__ void pipe_load(const StepArgs& a, unsigned row, unsigned stage, unsigned bar) {
+__device__ __forceinline__ void pipe_load(const StepArgs& a, unsigned row, unsigned stage, unsigned bar, L2Policy pol) {
     const int nx = a.geo.nx, ny = a.geo.ny, nz = a.geo.nz;
     const int y = static_cast<int>(row % static_cast<unsigned>(ny));
     const int z = static_cast<int>(row / static_cast<unsigned>(ny));
@@ -115,7 +115,7 @@ __device__ __forceinline__ void pipe_load(const StepArgs& a, unsigned row, unsig
         sz -= (sz >= nz) ? nz : 0;
         const T* src = static_cast<const T*>(a.fin) + (static_cast<unsigned>(lane) * static_cast<unsigned>(a.geo.pitch) +
                                                        static_cast<unsigned>((sz * ny + sy) * nx));
-        bulk_g2s(stage + static_cast<unsigned>(lane * CAP * sizeof(T)), src, bytes, bar);
+        bulk_g2s(stage + static_cast<unsigned>(lane * CAP * sizeof(T)), src, bytes, bar, pol);
     }
 }
 
@@ -211,8 +211,11 @@ __global__ void __launch_bounds__(CAP / 2 + 32, CAP > 256 ? 1 : (S == STORE_F32 
     unsigned long long* written = full + NS;
     unsigned char* stages = smem + 128;
     const unsigned stages_s = smem_addr(stages);
-    const int first = blockIdx.x, stride = gridDim.x;
-    const int mine = first < p.nrows ? (p.nrows - first + stride - 1) / stride : 0;
+    // rows blockIdx.x, blockIdx.x + gridDim.x, ... of the list, every other step from its end (what the last step
+    // wrote last is still in L2)
+    const int block = static_cast<int>(blockIdx.x), blocks = static_cast<int>(gridDim.x);
+    const int mine = block < p.nrows ? (p.nrows - block + blocks - 1) / blocks : 0;
+    const int first = a.reverse ? p.nrows - 1 - block : block, stride = a.reverse ? -blocks : blocks;
     if (threadIdx.x == 0) {
         for (int s = 0; s < NS; ++s) {
             mbar_init(smem_addr(&full[s]), 1);
@@ -223,10 +226,11 @@ __global__ void __launch_bounds__(CAP / 2 + 32, CAP > 256 ? 1 : (S == STORE_F32 
     __syncthreads();
     if (threadIdx.x >= NC) {
         // ---- producer warp: loads NS rows ahead, stores each row once its results are in place
+        const L2Policy pol = read_policy(a.evict_first);
         int issued = 0;  // rows whose loads have been issued (row r goes to stage r % NS)
         for (; issued < NS && issued < mine; ++issued)
             pipe_load<Q, CAP, T>(a, p.rows[first + issued * stride] & 0x0fffffffu, stages_s + issued * STAGE_B,
-                                 smem_addr(&full[issued]));
+                                 smem_addr(&full[issued]), pol);
         for (int it = 0; it < mine; ++it) {
             const int s = it % NS;
             const bool ok = mbar_wait(smem_addr(&written[s]), static_cast<unsigned>((it / NS) & 1));
@@ -243,7 +247,7 @@ __global__ void __launch_bounds__(CAP / 2 + 32, CAP > 256 ? 1 : (S == STORE_F32 
                 bulk_wait_read_0();  // this stage's stores have read it
                 __syncwarp();
                 pipe_load<Q, CAP, T>(a, p.rows[first + issued * stride] & 0x0fffffffu, stages_s + s * STAGE_B,
-                                     smem_addr(&full[s]));
+                                     smem_addr(&full[s]), pol);
                 ++issued;
             }
         }

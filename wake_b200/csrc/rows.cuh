@@ -1,8 +1,7 @@
 // Whole-row step kernel for the TRT lattices: one block per lattice row, two
 // adjacent nodes per thread.
 //
-// The pure-gather spans of k_step_fast carry their row in a table, so every
-// load address is built per thread from the row it reads. Here the block index
+// The cells of k_step_cells ignore the rows, so every load address there is built per node. Here the block index
 // is the row itself (z * ny + y): the row, its source rows and, for every
 // direction q, the element offset of the source row in plane q are the same for
 // all threads of the launch's block, and a load is that offset plus one of four
@@ -14,15 +13,15 @@
 //   cx = -1: node x reads x+1, node x+1 reads x+2 (wrapped to 0 at x = nx-2)
 //
 // and every direction's two results leave with one 32-bit (16-bit storage) or
-// 64-bit (FP32) streaming store. A row descriptor byte replaces the per-node
+// 64-bit (FP32) store. A row descriptor byte replaces the per-node
 // flag reads: ROW_FAST marks a row whose every node is a pure gather (no solid,
 // wall, curved link or momentum-exchange link in reach), with ROW_ZH_IN /
 // ROW_ZH_OUT when its first / last node is a Zou-He inlet / outlet. Other rows
-// exit at once; their pure-gather runs go to k_step_fast and the rest to k_step.
+// exit at once: k_step_cells steps them.
 //
 // Requirements (host-checked): TRT, nx even (rows start on a word boundary),
 // Q * pitch < 2^32 (32-bit element offsets), no coupled temperature. The per-node
-// arithmetic is trt_pairs2's, so results equal the span kernel's bit for bit.
+// arithmetic is trt_pairs2's, so results equal k_step_cells's bit for bit.
 #pragma once
 
 #include "stream_collide.cuh"
@@ -34,25 +33,25 @@ enum : uint8_t { ROW_FAST = 1u, ROW_ZH_IN = 2u, ROW_ZH_OUT = 4u };
 // Two adjacent populations of one plane (x even): a 64-bit word (FP32) or a 32-bit word of
 // two 16-bit values, as floats (node x in .x).
 template <int S>
-__device__ __forceinline__ float2 load_adjacent(const typename Codec<S>::T* p) {
+__device__ __forceinline__ float2 load_adjacent(const typename Codec<S>::T* p, L2Policy pol) {
     if constexpr (S == STORE_F32) {
         return __ldg(reinterpret_cast<const float2*>(p));
     } else if constexpr (S == STORE_F16C) {
-        return f16c_decode_word(__ldg(reinterpret_cast<const unsigned*>(p)));
+        return f16c_decode_word(ld_pop(reinterpret_cast<const unsigned*>(p), pol));
     } else {
-        const unsigned w = __ldg(reinterpret_cast<const unsigned*>(p));
+        const unsigned w = ld_pop(reinterpret_cast<const unsigned*>(p), pol);
         return make_float2(raw_lo<S>(w), raw_hi<S>(w));
     }
 }
 
 template <int S>
 __device__ __forceinline__ void store_adjacent(typename Codec<S>::T* p, float2 v) {
-    if constexpr (S == STORE_F32) __stcs(reinterpret_cast<float2*>(p), v);
+    if constexpr (S == STORE_F32) *reinterpret_cast<float2*>(p) = v;
     else store_pair<S>(p, v);
 }
 
 template <int Q, int S, bool LES>
-__global__ void __launch_bounds__(WK_FAST_MAX_THREADS, Q == 9 ? WK_FAST_TRT9_MIN_BLOCKS : WK_FAST_TRT_MIN_BLOCKS)
+__global__ void __launch_bounds__(WK_FAST_MAX_THREADS, Q == 9 ? 16 : 10)
     k_step_rows(const StepArgs a) {
     using L = Lat<Q>;
     using T = typename Codec<S>::T;
@@ -72,6 +71,7 @@ __global__ void __launch_bounds__(WK_FAST_MAX_THREADS, Q == 9 ? WK_FAST_TRT9_MIN
     const T* fin = static_cast<const T*>(a.fin);
     T* fout = static_cast<T*>(a.fout);
     const int lane = threadIdx.x & 31;
+    const L2Policy ld = read_policy(a.evict_first);
     for (int x0 = (threadIdx.x >> 5) * 64; x0 < nx; x0 += (blockDim.x >> 5) * 64) {
         const int xa = x0 + 2 * lane;  // nodes xa, xa + 1 (nx even: both in the row)
         if (xa >= nx) break;
@@ -81,9 +81,9 @@ __global__ void __launch_bounds__(WK_FAST_MAX_THREADS, Q == 9 ? WK_FAST_TRT9_MIN
 #pragma unroll
         for (int q = 0; q < Q; ++q) {
             const T* src = fin + (q * P + static_cast<unsigned>((zs[L::cz(q) + 1] * ny + ys[L::cy(q) + 1]) * nx));
-            if (L::cx(q) == 0) f[q] = load_adjacent<S>(src + xa);
-            else if (L::cx(q) > 0) f[q] = make_float2(load_raw<S>(src + xm), load_raw<S>(src + xa));
-            else f[q] = make_float2(load_raw<S>(src + (xa + 1)), load_raw<S>(src + xp));
+            if (L::cx(q) == 0) f[q] = load_adjacent<S>(src + xa, ld);
+            else if (L::cx(q) > 0) f[q] = make_float2(load_raw<S>(src + xm, ld), load_raw<S>(src + xa, ld));
+            else f[q] = make_float2(load_raw<S>(src + (xa + 1), ld), load_raw<S>(src + xp, ld));
         }
         if ((kind & ROW_ZH_IN) && xa == 0) zou_he_half<Q, HS>(f, 0, FL_ZH_IN, a.geo);
         if ((kind & ROW_ZH_OUT) && xa + 2 == nx) zou_he_half<Q, HS>(f, 1, FL_ZH_OUT, a.geo);

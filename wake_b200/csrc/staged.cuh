@@ -1,8 +1,7 @@
 // Persistent step kernel with the pure-gather rows staged in shared memory.
 //
-// Work of one step: the segments of the rows that are not entirely pure-gather
-// (walls, solids, curved links, momentum exchange; per-node path of step_chunk,
-// straight from global memory) and the pure-gather tiles. A tile is up to TILE_NODES nodes: `count` consecutive rows
+// Work of one launch: the pure-gather tiles; k_step_cells steps the other rows beside it. A tile is up to
+// TILE_NODES nodes: `count` consecutive rows
 // y0 .. y0+count-1 of one z plane, i.e. one contiguous range of node indices.
 // For direction q the tile's pull sources are the rows y0-cy .. y0-cy+count-1 of
 // plane z-cz: again one contiguous range of plane q (two when the range wraps
@@ -64,48 +63,23 @@ __device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity) {
     return false;
 }
 
-__device__ __forceinline__ void bulk_g2s(unsigned dst, const void* src, unsigned bytes, unsigned bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
-                 "l"(src), "r"(bytes), "r"(bar)
-                 : "memory");
+__device__ __forceinline__ void bulk_g2s(unsigned dst, const void* src, unsigned bytes, unsigned bar, L2Policy pol) {
+    asm volatile(
+        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;" ::"r"(
+            dst),
+        "l"(src), "r"(bytes), "r"(bar), "l"(pol)
+        : "memory");
 }
 
 __device__ __forceinline__ void fence_proxy_async_smem() {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
 
-// Work lists of one launch. tiles: (member, (z << 16) | y0, count, 0);
-// gen: (member, segment, entry, 0) for the general segments, entry = the
-// segment's index in its member's general-segment list (momentum-exchange
-// slots); spans: the pure-gather runs of the rows that hold general segments.
+// Tiles of one launch: (0, (z << 16) | y0, count, 0).
 struct TileArgs {
     const uint4* tiles;
     int ntiles;
-    const uint4* gen;
-    int ngen;
-    const BatchDom* dom;  // batch: member table; single lattice: null (the StepArgs parameter)
-    int parity;
-    const uint4* spans;   // pure-gather spans (member, row, x0, x1) of the rows outside the tiles
-    int nspans;
 };
-
-template <bool BATCH>
-__device__ __forceinline__ StepArgs tile_member(const StepArgs& a, const TileArgs& t, unsigned m) {
-    if constexpr (BATCH) {
-        const BatchDom* d = t.dom + m;
-        StepArgs r = d->a;
-        const int c = d->cur0 ^ t.parity;
-        r.fin = d->buf[c];
-        r.fout = d->buf[c ^ 1];
-        r.th.tin = d->tbuf[c];
-        r.th.tout = d->tbuf[c ^ 1];
-        return r;
-    } else {
-        (void)t;
-        (void)m;
-        return a;
-    }
-}
 
 // Issue the copies of one tile (warp 0): lane 0 posts the byte count, lane q
 // issues direction q's one or two copies.
@@ -116,6 +90,7 @@ __device__ __forceinline__ void tile_issue(const StepArgs& a, uint4 tl, unsigned
     const int y0 = static_cast<int>(tl.y & 0xffffu), z = static_cast<int>(tl.y >> 16), cnt = static_cast<int>(tl.z);
     const unsigned tile_b = static_cast<unsigned>(cnt * nx) * sizeof(T);
     const int lane = threadIdx.x & 31;
+    const L2Policy pol = read_policy(a.evict_first);
     if (lane == 0) mbar_expect_tx(bar, Q * tile_b);
     __syncwarp();
 #pragma unroll
@@ -131,8 +106,8 @@ __device__ __forceinline__ void tile_issue(const StepArgs& a, uint4 tl, unsigned
         const T* plane = static_cast<const T*>(a.fin) + static_cast<long long>(q) * a.geo.pitch;
         const unsigned dst = stage + static_cast<unsigned>(q) * (TILE_NODES * sizeof(T));
         const unsigned b1 = static_cast<unsigned>(first * nx) * sizeof(T);
-        bulk_g2s(dst, plane + (static_cast<long long>(sz) * ny + sy) * nx, b1, bar);
-        if (first < cnt) bulk_g2s(dst + b1, plane + static_cast<long long>(sz) * ny * nx, tile_b - b1, bar);
+        bulk_g2s(dst, plane + (static_cast<long long>(sz) * ny + sy) * nx, b1, bar, pol);
+        if (first < cnt) bulk_g2s(dst + b1, plane + static_cast<long long>(sz) * ny * nx, tile_b - b1, bar, pol);
     }
 }
 
@@ -170,12 +145,12 @@ __device__ __forceinline__ void tile_node_scalar(const StepArgs& a, const typena
     if (!(rho > 0.0f) || !(fabsf(u[0]) < 1e30f)) atomicOr(a.status, ERR_NONFINITE);
     T* out = static_cast<T*>(a.fout);
 #pragma unroll
-    for (int q = 0; q < Q; ++q) C::store_stream(out + (q * a.geo.pitch + base + n), f[q], L::w(q));
+    for (int q = 0; q < Q; ++q) store_f<S>(out + (q * a.geo.pitch + base + n), f[q], L::w(q));
 }
 
-// Nodes n and n + TILE_THREADS of a tile, TRT in packed FP32 (h-space for shifted storage).
-template <int Q, int S, bool LES>
-__device__ __forceinline__ void tile_pair_trt(const StepArgs& a, const typename Codec<S>::T* st, long long base,
+// Nodes n and n + TILE_THREADS of a tile, in packed FP32 (h-space for shifted storage).
+template <int Q, int COLL, int S, bool LES>
+__device__ __forceinline__ void tile_pair(const StepArgs& a, const typename Codec<S>::T* st, long long base,
                                               int na, int count_nodes, int nx) {
     using L = Lat<Q>;
     using T = typename Codec<S>::T;
@@ -198,7 +173,8 @@ __device__ __forceinline__ void tile_pair_trt(const StepArgs& a, const typename 
         if (fb & (FL_ZH_IN | FL_ZH_OUT)) zou_he_half<Q, HS>(f, 1, fb, a.geo);
     }
     float2 rho, u[3];
-    trt_pairs2<Q, LES, HS>(f, a.phys, rho, u);
+    collide_pairs2<Q, COLL, S, LES>(f, a.phys, bc2(a.phys.g[1]),
+                                    a.phys.g[0] != 0.0f || a.phys.g[1] != 0.0f || a.phys.g[2] != 0.0f, rho, u);
     const bool bad =
         !(rho.x > 0.0f) || !(fabsf(u[0].x) < 1e30f) || (vb && (!(rho.y > 0.0f) || !(fabsf(u[0].y) < 1e30f)));
     if (bad) atomicOr(a.status, ERR_NONFINITE);
@@ -210,8 +186,8 @@ __device__ __forceinline__ void tile_pair_trt(const StepArgs& a, const typename 
     }
 }
 
-template <int Q, int COLL, int S, bool LES, bool BATCH>
-__global__ void __launch_bounds__(TILE_THREADS, TILE_CTAS_PER_SM) k_step_tiles(const StepArgs a0, const TileArgs t) {
+template <int Q, int COLL, int S, bool LES>
+__global__ void __launch_bounds__(TILE_THREADS, TILE_CTAS_PER_SM) k_step_tiles(const StepArgs a, const TileArgs t) {
     using T = typename Codec<S>::T;
     constexpr unsigned STAGE_B = Q * TILE_NODES * sizeof(T);
     extern __shared__ __align__(128) unsigned char smem[];
@@ -226,32 +202,12 @@ __global__ void __launch_bounds__(TILE_THREADS, TILE_CTAS_PER_SM) k_step_tiles(c
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
-    // the first tiles' copies go out before the general rows, so they land meanwhile
-    if (issuer) {
-        for (int k = 0; k < TILE_STAGES && k < mine; ++k) {
-            const uint4 tl = t.tiles[first + k * stride];
-            tile_issue<Q, T>(tile_member<BATCH>(a0, t, tl.x), tl, stages_s + k * STAGE_B, smem_addr(&bars[k]));
-        }
-    }
-    // rows outside the tiles, from global memory: general segments one warp per
-    // 32-node chunk, pure-gather spans one CTA per span (the direct kernels' paths)
-    {
-        const int warps = blockDim.x >> 5;
-        constexpr int CPS = SEG / 32;  // warp chunks per segment
-        for (int g = first * warps + static_cast<int>(threadIdx.x >> 5); g < CPS * t.ngen; g += stride * warps) {
-            const uint4 r = t.gen[g / CPS];
-            step_chunk<Q, COLL, S, LES>(tile_member<BATCH>(a0, t, r.x), r.y, static_cast<int>(r.z), g % CPS);
-        }
-        for (int sp = first; sp < t.nspans; sp += stride) {
-            const uint4 r = t.spans[sp];
-            const StepArgs a = tile_member<BATCH>(a0, t, r.x);
-            step_span_fast<Q, COLL, S, LES, false>(a, span_decode(r, a.geo));
-        }
-    }
+    if (issuer)
+        for (int k = 0; k < TILE_STAGES && k < mine; ++k)
+            tile_issue<Q, T>(a, t.tiles[first + k * stride], stages_s + k * STAGE_B, smem_addr(&bars[k]));
     for (int it = 0; it < mine; ++it) {
         const int s = it % TILE_STAGES;
         const uint4 tl = t.tiles[first + it * stride];
-        const StepArgs a = tile_member<BATCH>(a0, t, tl.x);
         const bool ok = mbar_wait(smem_addr(&bars[s]), static_cast<unsigned>((it / TILE_STAGES) & 1));
         if (!__syncthreads_and(ok)) {
             if (threadIdx.x == 0) atomicOr(a.status, ERR_STAGE_TIMEOUT);
@@ -264,9 +220,9 @@ __global__ void __launch_bounds__(TILE_THREADS, TILE_CTAS_PER_SM) k_step_tiles(c
         const int y0 = static_cast<int>(tl.y & 0xffffu), z = static_cast<int>(tl.y >> 16);
         const int count_nodes = static_cast<int>(tl.z) * nx;
         const long long base = (static_cast<long long>(z) * a.geo.ny + y0) * nx;
-        if constexpr (COLL == COLL_TRT) {
+        if constexpr (pure_pairs<Q, COLL, S>()) {
             if (static_cast<int>(threadIdx.x) < count_nodes)
-                tile_pair_trt<Q, S, LES>(a, st, base, threadIdx.x, count_nodes, nx);
+                tile_pair<Q, COLL, S, LES>(a, st, base, threadIdx.x, count_nodes, nx);
         } else {
             for (int n = threadIdx.x; n < count_nodes; n += TILE_THREADS)
                 tile_node_scalar<Q, COLL, S, LES>(a, st, base, n, nx);
@@ -275,7 +231,7 @@ __global__ void __launch_bounds__(TILE_THREADS, TILE_CTAS_PER_SM) k_step_tiles(c
         if (issuer && it + TILE_STAGES < mine) {
             fence_proxy_async_smem();
             const uint4 tn = t.tiles[first + (it + TILE_STAGES) * stride];
-            tile_issue<Q, T>(tile_member<BATCH>(a0, t, tn.x), tn, stages_s + s * STAGE_B, smem_addr(&bars[s]));
+            tile_issue<Q, T>(a, tn, stages_s + s * STAGE_B, smem_addr(&bars[s]));
         }
     }
 }

@@ -135,18 +135,14 @@ def hbm_peak():
     return FALLBACK_HBM_GBS, "fallback"
 
 
-KERNEL_NAMES = {1: ("wk::k_step_fast<19, TRT, {S}, LES, IDX32>", "spans"), 3: ("wk::k_step_rows<19, {S}, LES>", "rows"),
+KERNEL_NAMES = {1: ("wk::k_step_cells<19, TRT, {S}, LES>", "cells"), 3: ("wk::k_step_rows<19, {S}, LES>", "rows"),
                 4: ("wk::k_step_rows_pipe<19, {S}, LES, 256>", "pipe")}
 
 
 def bulk_bytes_per_node(g, storage):
-    """Algorithmic DRAM bytes per node of the D3Q19 bulk launch: 19 populations read and 19
-    written, plus the node's flag byte for the span and tile kernels (variants 1, 2); the
-    whole-row kernels read one descriptor byte per row instead (under 0.01 B per node)."""
-    import wake_b200 as wb
-
-    flag = 1 if wb.lib.wake_grid_get_kernel(g.handle) in (1, 2) else 0
-    return 2 * 19 * (4 if storage == "f32" else 2) + flag
+    """Algorithmic DRAM bytes per node of the D3Q19 bulk launch: 19 populations read and 19 written (the
+    class bytes of the cells or rows, one per 64 nodes or per row, are under 0.02 B per node)."""
+    return 2 * 19 * (4 if storage == "f32" else 2)
 
 
 def bulk_kernel(g, storage):

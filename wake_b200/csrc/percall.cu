@@ -156,54 +156,90 @@ __global__ void k_collide(const float* __restrict__ fin, float* __restrict__ fou
     for (int q = 0; q < Q; ++q) fout[q * n + i] = f[q];
 }
 
-// Fully periodic pull (d2q9_streaming.ispc:4-29, d3q19_streaming.ispc:4-35, d3q27_streaming.ispc:4-35).
-template <int Q>
-__global__ void k_stream_periodic(const float* __restrict__ src, float* __restrict__ dst, int nx, int ny, int nz) {
-    using L = Lat<Q>;
-    const long long n = static_cast<long long>(nx) * ny * nz;
-    const long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
-    if (i >= n) return;
-    const int x = static_cast<int>(i % nx), y = static_cast<int>((i / nx) % ny), z = static_cast<int>(i / (static_cast<long long>(nx) * ny));
-#pragma unroll
-    for (int q = 0; q < Q; ++q) {
-        const int sx = wrap<Q>(x - L::cx(q), nx), sy = wrap<Q>(y - L::cy(q), ny), sz = wrap<Q>(z - L::cz(q), nz);
-        dst[q * n + i] = src[q * n + (static_cast<long long>(sz) * ny + sy) * nx + sx];
+// Lattice sizes with what turns a node index into coordinates: 32-bit multiplications for up to 2^31 nodes (WIDE =
+// false), 64-bit divisions above, which cost a node as much as its memory traffic.
+struct Box {
+    int nx, ny, nz;
+    FastDiv by_nx, by_ny;
+    long long n;
+};
+Box box_of(int nx, int ny, int nz) {
+    return {nx, ny, nz, FastDiv::of(static_cast<unsigned>(nx)), FastDiv::of(static_cast<unsigned>(ny)),
+            static_cast<long long>(nx) * ny * nz};
+}
+inline bool wide(long long n) { return n > 0x7fffffffll; }
+template <bool WIDE>
+__device__ __forceinline__ void node_at(const Box& b, long long i, int& x, int& y, int& z) {
+    if (WIDE) {
+        x = static_cast<int>(i % b.nx);
+        y = static_cast<int>((i / b.nx) % b.ny);
+        z = static_cast<int>(i / (static_cast<long long>(b.nx) * b.ny));
+    } else {
+        const unsigned u = static_cast<unsigned>(i), row = b.by_nx.quot(u), k = b.by_ny.quot(row);
+        x = static_cast<int>(u - row * b.nx);
+        y = static_cast<int>(row - k * b.ny);
+        z = static_cast<int>(k);
     }
 }
 
-// Pull with half-way bounce-back (d2q9_streaming.ispc:33-95, d3q19_streaming.ispc:39-104).
-template <int Q>
-__global__ void k_stream_bounded(const float* __restrict__ src, float* __restrict__ dst, const uint8_t* __restrict__ ct,
-                                 int nx, int ny, int nz, float uwx, float uwy, float uwz) {
+// Fully periodic pull (d2q9_streaming.ispc:4-29, d3q19_streaming.ispc:4-35, d3q27_streaming.ispc:4-35).
+template <int Q, bool WIDE>
+__global__ void __launch_bounds__(256) k_stream_periodic(const float* __restrict__ src, float* __restrict__ dst, const Box b) {
     using L = Lat<Q>;
-    const long long n = static_cast<long long>(nx) * ny * nz;
     const long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
-    if (i >= n) return;
-    const int x = static_cast<int>(i % nx), y = static_cast<int>((i / nx) % ny), z = static_cast<int>(i / (static_cast<long long>(nx) * ny));
-    const bool solid = ct[i] == CT_SOLID;
+    if (i >= b.n) return;
+    int x, y, z;
+    node_at<WIDE>(b, i, x, y, z);
 #pragma unroll
     for (int q = 0; q < Q; ++q) {
-        if (solid) {
-            dst[q * n + i] = src[q * n + i];
-            continue;
-        }
-        const int o = L::opp(q);
-        const int sx = wrap<Q>(x - L::cx(q), nx), sy = y - L::cy(q), sz = z - L::cz(q);
-        if (sy >= 0 && sy < ny && sz >= 0 && sz < nz) {
-            const long long s = (static_cast<long long>(sz) * ny + sy) * nx + sx;
-            const uint8_t t = ct[s];
-            if (t == CT_SOLID) {
-                dst[q * n + i] = src[o * n + i];
-            } else if (t == CT_MOVING_WALL) {
-                const float ci_uw = float(L::cx(q)) * uwx + float(L::cy(q)) * uwy + float(L::cz(q)) * uwz;
-                dst[q * n + i] = src[o * n + i] + 2.0f * L::w(q) * 1.0f * 3.0f * ci_uw;
-            } else {
-                dst[q * n + i] = src[q * n + s];
-            }
+        const int sx = wrap<Q>(x - L::cx(q), b.nx), sy = wrap<Q>(y - L::cy(q), b.ny), sz = wrap<Q>(z - L::cz(q), b.nz);
+        dst[q * b.n + i] = src[q * b.n + (static_cast<long long>(sz) * b.ny + sy) * b.nx + sx];
+    }
+}
+
+// Pull with half-way bounce-back (d2q9_streaming.ispc:33-95, d3q19_streaming.ispc:39-104). The neighbours' types are
+// read first, then every population from where they say, so a node waits for memory twice and not once per direction.
+template <int Q, bool WIDE>
+__global__ void __launch_bounds__(256) k_stream_bounded(const float* __restrict__ src, float* __restrict__ dst,
+                                                        const uint8_t* __restrict__ ct, const Box b, float uwx, float uwy,
+                                                        float uwz) {
+    using L = Lat<Q>;
+    const long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
+    if (i >= b.n) return;
+    int x, y, z;
+    node_at<WIDE>(b, i, x, y, z);
+    const bool solid = ct[i] == CT_SOLID;
+    unsigned back = 0, moving = 0;
+#pragma unroll
+    for (int q = 1; q < Q; ++q) {
+        const int sx = wrap<Q>(x - L::cx(q), b.nx), sy = y - L::cy(q), sz = z - L::cz(q);
+        if (sy >= 0 && sy < b.ny && sz >= 0 && sz < b.nz) {
+            const uint8_t t = ct[i + (static_cast<long long>(sz - z) * b.ny + (sy - y)) * b.nx + (sx - x)];
+            if (t == CT_SOLID || t == CT_MOVING_WALL) back |= 1u << q;
+            if (t == CT_MOVING_WALL) moving |= 1u << q;
         } else {
-            dst[q * n + i] = src[o * n + i];
+            back |= 1u << q;
         }
     }
+    float f[Q];
+    f[0] = src[i];
+#pragma unroll
+    for (int q = 1; q < Q; ++q) {
+        const int sx = wrap<Q>(x - L::cx(q), b.nx);
+        const float* p = src + q * b.n + i + (-static_cast<long long>(L::cz(q)) * b.ny - L::cy(q)) * b.nx + (sx - x);
+        if ((back >> q) & 1u) p = src + L::opp(q) * b.n + i;
+        if (solid) p = src + q * b.n + i;
+        f[q] = *p;
+    }
+    if (moving && !solid) {
+#pragma unroll
+        for (int q = 1; q < Q; ++q) {
+            const float ci_uw = float(L::cx(q)) * uwx + float(L::cy(q)) * uwy + float(L::cz(q)) * uwz;
+            if ((moving >> q) & 1u) f[q] = f[q] + 2.0f * L::w(q) * 1.0f * 3.0f * ci_uw;
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < Q; ++q) dst[q * b.n + i] = f[q];
 }
 
 // In-place full-way swap on solid / moving-wall nodes (d2q9_boundaries.ispc:5-39).
@@ -303,18 +339,25 @@ __global__ void k_speed(const float* ux, const float* uy, const float* uz, float
 }
 
 // Momentum exchange (forces_momentum_exchange.ispc:6-138), FP64 block partials.
-template <int Q>
-__global__ void k_mem_partials(const float* __restrict__ f, const uint8_t* __restrict__ ct, int nx, int ny, int nz,
-                               float cx, float cy, float cz, float rmax, double* __restrict__ part) {
+template <int Q, bool WIDE>
+__global__ void __launch_bounds__(256) k_mem_partials(const float* __restrict__ f, const uint8_t* __restrict__ ct, const Box b,
+                                                      float cx, float cy, float cz, float rmax, double* __restrict__ part) {
     using L = Lat<Q>;
     __shared__ double red[3][256];
-    const long long n = static_cast<long long>(nx) * ny * nz;
+    const long long n = b.n;
+    const int nx = b.nx, ny = b.ny, nz = b.nz;
     double acc[3] = {0.0, 0.0, 0.0};
     const float rmax_sq = rmax * rmax;
+    // No link of a node further than rmax + 1 from the centre is in reach (links are within 0.87 of it; the small
+    // multiples of rmax and of the coordinates cover the roundings): its neighbours' types need not be read.
+    const float slack = 1e-4f * rmax + 1e-6f * (fabsf(cx) + fabsf(cy) + fabsf(cz) + float(nx) + float(ny) + float(nz));
+    const float far = rmax > 0.0f ? rmax + 1.0f + slack : __int_as_float(0x7f800000);
     for (long long i = blockIdx.x * 256ll + threadIdx.x; i < n; i += 256ll * gridDim.x) {
         if (ct[i] != CT_FLUID) continue;
-        const int x = static_cast<int>(i % nx), y = static_cast<int>((i / nx) % ny),
-                  z = static_cast<int>(i / (static_cast<long long>(nx) * ny));
+        int x, y, z;
+        node_at<WIDE>(b, i, x, y, z);
+        const float ox = float(x) - cx, oy = float(y) - cy, oz = L::D == 3 ? float(z) - cz : 0.0f;
+        if (ox * ox + oy * oy + oz * oz > far * far) continue;
 #pragma unroll
         for (int q = 1; q < Q; ++q) {
             const int xn = wrap<Q>(x + L::cx(q), nx), yn = y + L::cy(q), zn = z + L::cz(q);
@@ -345,14 +388,23 @@ __global__ void k_mem_partials(const float* __restrict__ f, const uint8_t* __res
         for (int c = 0; c < 3; ++c) part[3 * blockIdx.x + c] = red[c][0];
 }
 
-__global__ void k_mem_final(const double* part, int nblocks, float* o0, float* o1, float* o2) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+// One block: 256 strided sums and a fixed tree.
+__global__ void __launch_bounds__(256) k_mem_final(const double* part, int nblocks, float* o0, float* o1, float* o2) {
+    __shared__ double red[3][256];
     double s[3] = {0.0, 0.0, 0.0};
-    for (int b = 0; b < nblocks; ++b)
+    for (int b = threadIdx.x; b < nblocks; b += 256)
         for (int c = 0; c < 3; ++c) s[c] += part[3 * b + c];
-    *o0 = static_cast<float>(s[0]);
-    *o1 = static_cast<float>(s[1]);
-    *o2 = static_cast<float>(s[2]);
+    for (int c = 0; c < 3; ++c) red[c][threadIdx.x] = s[c];
+    __syncthreads();
+    for (int o = 128; o > 0; o >>= 1) {
+        if (threadIdx.x < o)
+            for (int c = 0; c < 3; ++c) red[c][threadIdx.x] += red[c][threadIdx.x + o];
+        __syncthreads();
+    }
+    if (threadIdx.x != 0) return;
+    *o0 = static_cast<float>(red[0][0]);
+    *o1 = static_cast<float>(red[1][0]);
+    *o2 = static_cast<float>(red[2][0]);
 }
 
 // BFL (d3q19_curved.ispc:7-71), one thread per link.
@@ -462,6 +514,12 @@ void collide_call(const float* fin, float* fout, const uint8_t* ct, float* rho, 
 }
 
 template <int Q>
+void mem_partials(int nb, const float* f, const uint8_t* ct, const Box& b, float cx, float cy, float cz, float rmax, double* part) {
+    if (wide(b.n)) k_mem_partials<Q, true><<<nb, 256>>>(f, ct, b, cx, cy, cz, rmax, part);
+    else k_mem_partials<Q, false><<<nb, 256>>>(f, ct, b, cx, cy, cz, rmax, part);
+}
+
+template <int Q>
 void mem_call(const float* f, const uint8_t* ct, int nx, int ny, int nz, float cx, float cy, float cz, float rmax,
               float* o0, float* o1, float* o2) {
     const long long n = static_cast<long long>(nx) * ny * nz;
@@ -479,9 +537,9 @@ void mem_call(const float* f, const uint8_t* ct, int nx, int ny, int nz, float c
         set_error(WAKE_ERR_NOMEM, "momentum exchange: partials");
         return;
     }
-    k_mem_partials<Q><<<nb, 256>>>(s.ptr<float>(0), s.ptr<uint8_t>(1), nx, ny, nz, cx, cy, cz, rmax, part.as<double>());
-    k_mem_final<<<1, 32>>>(part.as<double>(), nb, s.ptr<float>(2), s.ptr<float>(3), s.ptr<float>(4));
-    s.end();
+    mem_partials<Q>(nb, s.ptr<float>(0), s.ptr<uint8_t>(1), box_of(nx, ny, nz), cx, cy, cz, rmax, part.as<double>());
+    k_mem_final<<<1, 256>>>(part.as<double>(), nb, s.ptr<float>(2), s.ptr<float>(3), s.ptr<float>(4));
+    if (s.end() == WAKE_OK) part.release();  // to the block cache: a cudaFree costs more than the kernels
 }
 
 }  // namespace
@@ -529,9 +587,11 @@ static void stream_periodic_call(int Q, const float* src, float* dst, int nx, in
     s.out(dst, Q * static_cast<std::size_t>(n));
     if (s.begin()) return;
     const int nb = blocks_for(n);
-    if (Q == 9) k_stream_periodic<9><<<nb, 256>>>(s.ptr<float>(0), s.ptr<float>(1), nx, ny, nz);
-    else if (Q == 19) k_stream_periodic<19><<<nb, 256>>>(s.ptr<float>(0), s.ptr<float>(1), nx, ny, nz);
-    else k_stream_periodic<27><<<nb, 256>>>(s.ptr<float>(0), s.ptr<float>(1), nx, ny, nz);
+    const Box b = box_of(nx, ny, nz);
+    const auto go = [&](auto kernel) { kernel<<<nb, 256>>>(s.ptr<float>(0), s.ptr<float>(1), b); };
+    if (Q == 9) wide(n) ? go(k_stream_periodic<9, true>) : go(k_stream_periodic<9, false>);
+    else if (Q == 19) wide(n) ? go(k_stream_periodic<19, true>) : go(k_stream_periodic<19, false>);
+    else wide(n) ? go(k_stream_periodic<27, true>) : go(k_stream_periodic<27, false>);
     s.end();
 }
 void d2q9_stream_periodic(const float f_src[], float f_dst[], int nx, int ny) {
@@ -554,8 +614,12 @@ static void stream_bounded_call(int Q, const float* src, float* dst, const uint8
     s.in(ct, static_cast<std::size_t>(n));
     if (s.begin()) return;
     const int nb = blocks_for(n);
-    if (Q == 9) k_stream_bounded<9><<<nb, 256>>>(s.ptr<float>(0), s.ptr<float>(1), s.ptr<uint8_t>(2), nx, ny, nz, uwx, uwy, 0.f);
-    else k_stream_bounded<19><<<nb, 256>>>(s.ptr<float>(0), s.ptr<float>(1), s.ptr<uint8_t>(2), nx, ny, nz, uwx, uwy, uwz);
+    const Box b = box_of(nx, ny, nz);
+    const auto go = [&](auto kernel) {
+        kernel<<<nb, 256>>>(s.ptr<float>(0), s.ptr<float>(1), s.ptr<uint8_t>(2), b, uwx, uwy, Q == 9 ? 0.f : uwz);
+    };
+    if (Q == 9) wide(n) ? go(k_stream_bounded<9, true>) : go(k_stream_bounded<9, false>);
+    else wide(n) ? go(k_stream_bounded<19, true>) : go(k_stream_bounded<19, false>);
     s.end();
 }
 void d2q9_stream_with_boundaries(const float f_src[], float f_dst[], const uint8_t cell_type[], int nx, int ny,
@@ -772,10 +836,9 @@ extern "C" int d3q19_compute_momentum_exchange_forces_noalloc(const float f_post
     // one block per 256 nodes, so each block writes its own partial before the
     // final kernel reads it: nothing from an earlier call is read back
     const int nb = static_cast<int>((n + 255) / 256);
-    k_mem_partials<19><<<nb, 256>>>(f_post_collision, cell_type, nx, ny, nz, center_x, center_y, center_z, max_radius,
-                                     part);
+    mem_partials<19>(nb, f_post_collision, cell_type, box_of(nx, ny, nz), center_x, center_y, center_z, max_radius, part);
     WK_CUDA(cudaGetLastError());
-    k_mem_final<<<1, 32>>>(part, nb, fx_out, fy_out, fz_out);
+    k_mem_final<<<1, 256>>>(part, nb, fx_out, fy_out, fz_out);
     WK_CUDA(cudaGetLastError());
     WK_CUDA(cudaStreamSynchronize(0));
     return WAKE_OK;

@@ -895,6 +895,7 @@ int do_steps(wake_grid* g, int n) {
         const bool bulk = by_rows && g->n_row_fast > 0;
         const bool beside = !by_rows || !g->rest.units.empty() || g->mem_on;
         const bool fork = bulk && beside;
+        a.early = !fork;  // (a launch on the forked stream follows an event)
         if (fork) {
             WK_CUDA(cudaEventRecord(g->ev_fork, g->stream));
             WK_CUDA(cudaStreamWaitEvent(g->side, g->ev_fork, 0));

@@ -193,17 +193,32 @@ unsigned plan(unsigned units, int tpb, unsigned list_blocks, unsigned& run, unsi
     return blocks;
 }
 
+// Launch a step kernel; early: it may start before the kernel before it on the stream has ended (after_last_step).
+template <class A>
+void launch_step(void (*kernel)(A), unsigned blocks, int tpb, cudaStream_t st, const A& a, bool early) {
+    cudaLaunchConfig_t c{};
+    c.gridDim = dim3(blocks);
+    c.blockDim = dim3(static_cast<unsigned>(tpb));
+    c.stream = st;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = &at;
+    c.numAttrs = early ? 1 : 0;
+    (void)cudaLaunchKernelEx(&c, kernel, a);  // the caller reads the error
+}
+
 template <int C, int S, bool LES, bool TH>
 void cells_one(StepArgs& a, int tpb, cudaStream_t st) {
     a.list_blocks = blocks_of(a.nunits + (a.mem.enabled ? 1u : 0u), tpb);
     const unsigned blocks = plan(a.cells * pure_units<kQ, C, S, TH>(), tpb, a.list_blocks, a.run, a.spread);
-    if (blocks) k_step_cells<kQ, C, S, LES, TH><<<blocks, tpb, 0, st>>>(a);
+    if (blocks) launch_step(k_step_cells<kQ, C, S, LES, TH>, blocks, tpb, st, a, a.early != 0);
 }
 template <int C, int S, bool LES, bool TH>
 void batch_one(BatchArgs& b, int tpb, cudaStream_t st) {
     b.list_blocks = blocks_of(b.nlisted, tpb);
     const unsigned blocks = plan(b.npure * pure_units<kQ, C, S, false>(), tpb, b.list_blocks, b.run, b.spread);
-    if (blocks) k_step_cells_batch<kQ, C, S, LES, TH><<<blocks, tpb, 0, st>>>(b);
+    if (blocks) launch_step(k_step_cells_batch<kQ, C, S, LES, TH>, blocks, tpb, st, b, true);
 }
 template <int C, int S, bool LES>
 void initial_one(const float* f0, void* A, void* B, const uint8_t* flags, const Geo& g, const Physics& p,

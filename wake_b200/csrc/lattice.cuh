@@ -29,19 +29,21 @@ __device__ __forceinline__ L2Policy read_policy(bool evict_first) {
     asm("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(normal));
     return evict_first ? first : normal;
 }
+// (Not the read-only path: a step kernel may be resident while the step before it still writes what it will read,
+// and volatile keeps the loads behind the wait for it, after_last_step.)
 __device__ __forceinline__ float ld_pop(const float* p, L2Policy pol) {
     float v;
-    asm("ld.global.nc.L2::cache_hint.f32 %0, [%1], %2;" : "=f"(v) : "l"(p), "l"(pol));
+    asm volatile("ld.global.L2::cache_hint.f32 %0, [%1], %2;" : "=f"(v) : "l"(p), "l"(pol));
     return v;
 }
 __device__ __forceinline__ unsigned ld_pop(const unsigned* p, L2Policy pol) {
     unsigned v;
-    asm("ld.global.nc.L2::cache_hint.u32 %0, [%1], %2;" : "=r"(v) : "l"(p), "l"(pol));
+    asm volatile("ld.global.L2::cache_hint.u32 %0, [%1], %2;" : "=r"(v) : "l"(p), "l"(pol));
     return v;
 }
 __device__ __forceinline__ unsigned short ld_pop(const unsigned short* p, L2Policy pol) {
     unsigned short v;
-    asm("ld.global.nc.L2::cache_hint.u16 %0, [%1], %2;" : "=h"(v) : "l"(p), "l"(pol));
+    asm volatile("ld.global.L2::cache_hint.u16 %0, [%1], %2;" : "=h"(v) : "l"(p), "l"(pol));
     return v;
 }
 

@@ -286,6 +286,7 @@ struct StepArgs {
     unsigned run;             // units per warp of the direct range
     int reverse;              // the sweep runs from the lattice's end (every other step)
     int evict_first;          // policy of the population loads (read_policy)
+    int early;                // host: the launch may start before the stream's last kernel has ended (launch_step)
     unsigned nunits, list_blocks, spread;
     const unsigned* units;    // units of the listed cells (cells.cuh)
     const uint4* list;        // listed cells: first node, node count | LIST_* bits, first curved link, links

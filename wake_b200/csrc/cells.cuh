@@ -561,13 +561,13 @@ __device__ __forceinline__ unsigned which_block(unsigned list_blocks, unsigned s
     return first ? k : (reverse ? gridDim.x - list_blocks - 1u - pb : pb);
 }
 
-// A step's launch may start before the step before it has ended (launch_step): wait for that one's results, then let
-// the next one start. Its blocks come up under this step's last ones, wait and take over, where they had the latency
-// of a launch between steps: D2Q9 400x160 in a graph 2.95 -> 2.53 us a step, as plain launches 4.1 -> 2.5 (the host's
-// rate of launches), with a temperature 384x192 5.6 -> 4.0; D3Q19 48^3 sphere 5.9 -> 5.5, 256x128x128 109.9 -> 109.6.
+// A step's launch may start before the step before it has ended (launch_step), as that one's blocks end: wait for its
+// results. The blocks come up and take over where they had the latency of a launch between steps: D2Q9
+// 400x160 in a graph 2.95 -> 2.5 us a step, as plain launches 4.1 -> 2.5 (the host's rate of launches), with a
+// temperature 384x192 5.6 -> 4.0; D3Q19 48^3 sphere 5.9 -> 5.5, 256x128x128 109.9 -> 109.6. Letting the next launch
+// start as soon as every block of this one runs was slower (1024x512 BGK 9.4 / 8.6, temperature 3.2 / 3.0 in graphs).
 __device__ __forceinline__ void after_last_step() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
 // One step of one lattice: the listed cells and the pure cells of cells 0 .. cells - 1.

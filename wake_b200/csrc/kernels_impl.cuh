@@ -183,10 +183,11 @@ unsigned blocks_of(unsigned units, int tpb) {
 // Blocks of a launch over `units` pure units, and how they are laid out. Two units per warp where the blocks
 // still fill the device (148 SMs, 10 or more blocks each) several times over: a block's start costs about a tenth
 // of a one-unit block's life (D3Q19 FP32 160^3: 110.5 us with one, 106.6 with two, 113 with eight); smaller
-// lattices need the blocks to even out the end (97^3: 27.3 / 26.8 / 29.8).
+// lattices need the blocks to even out the end (97^3: 27.3 / 26.8 / 29.8; D2Q9 1024x512, 8192 blocks of one unit: BGK
+// 9.4 / 8.5, MRT 9.0 / 7.5).
 unsigned plan(unsigned units, int tpb, unsigned list_blocks, unsigned& run, unsigned& spread) {
     unsigned blocks = blocks_of(units, tpb);
-    run = blocks >= 148u * 64u ? 2u : 1u;
+    run = blocks >= 148u * 40u ? 2u : 1u;
     blocks = list_blocks + (blocks + run - 1u) / run;
     spread = 0;
     while (list_blocks && (static_cast<unsigned long long>(list_blocks) << (spread + 1)) <= blocks / 5ull * 3ull) ++spread;

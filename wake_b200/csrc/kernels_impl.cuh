@@ -153,7 +153,7 @@ __global__ void __launch_bounds__(512) k_direct(const void* fin_v, const uint8_t
 #pragma unroll
         for (int q = 0; q < Q; ++q) out.f[q * geo.pitch + i] = f[q];
     }
-    if (out.rho) {
+    if (out.macro) {
         float g[3] = {phys.g[0], phys.g[1], phys.g[2]};
         if (th.on) {  // local buoyancy of the state's temperature (sum of the current temperature buffer)
             float t5[5];
@@ -163,11 +163,7 @@ __global__ void __launch_bounds__(512) k_direct(const void* fin_v, const uint8_t
         }
         float rho, u[3];
         node_moments<Q>(f, g, rho, u);
-        out.rho[i] = rho;
-        out.ux[i] = u[0];
-        out.uy[i] = u[1];
-        if (out.uz) out.uz[i] = u[2];
-        out.speed[i] = sqrtf(u[0] * u[0] + u[1] * u[1] + u[2] * u[2]);
+        store_macro(out, i, rho, u);
     }
     (void)flags;
 }

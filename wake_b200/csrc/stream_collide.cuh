@@ -77,14 +77,22 @@ struct MemCfg {                   // momentum-exchange monitor
     int hist_cap;
 };
 
-struct Out {                      // optional outputs of the materialise kernel
+struct Out {                      // optional outputs of the materialise kernel, null for those not wanted
     float* f;                     // FP32 f^k planes (pitch as the state buffers)
+    int macro;                    // some moment is wanted
     float* rho;
     float* ux;
     float* uy;
     float* uz;
     float* speed;
 };
+__device__ __forceinline__ void store_macro(const Out& out, long long i, float rho, const float u[3]) {
+    if (out.rho) out.rho[i] = rho;
+    if (out.ux) out.ux[i] = u[0];
+    if (out.uy) out.uy[i] = u[1];
+    if (out.uz) out.uz[i] = u[2];
+    if (out.speed) out.speed[i] = sqrtf(u[0] * u[0] + u[1] * u[1] + u[2] * u[2]);
+}
 
 template <int Q>
 __device__ __forceinline__ int wrap(int v, int n) {
@@ -411,7 +419,7 @@ __global__ void __launch_bounds__(512) k_materialise(const void* fin_v, const ui
 #pragma unroll
         for (int q = 0; q < Q; ++q) out.f[q * geo.pitch + i] = f[q];
     }
-    if (out.rho) {
+    if (out.macro) {
         float g[3] = {phys.g[0], phys.g[1], phys.g[2]};
         if (th.on) {  // the step's local buoyancy: T^k is the sum of the current post-collision temperature
             float t5[5];
@@ -421,11 +429,7 @@ __global__ void __launch_bounds__(512) k_materialise(const void* fin_v, const ui
         }
         float rho, u[3];
         node_moments<Q>(f, g, rho, u);
-        out.rho[i] = rho;
-        out.ux[i] = u[0];
-        out.uy[i] = u[1];
-        if (out.uz) out.uz[i] = u[2];
-        out.speed[i] = sqrtf(u[0] * u[0] + u[1] * u[1] + u[2] * u[2]);
+        store_macro(out, i, rho, u);
     }
 }
 

@@ -71,7 +71,7 @@ def parse():
                         "('vorticity': --steps calls of the 3D vorticity / Q-criterion kernel on 256^3 device fields)")
     p.add_argument("--block", type=int, default=0, help="threads per block of the fused step (0: automatic)")
     p.add_argument("--kernel", type=int, default=0,
-                   help="pure-gather kernel: 0 auto, 1 spans, 2 staged tiles, 3 whole rows, 4 pipelined whole rows")
+                   help="pure-gather kernel: 0 auto, 1 cells, 2 staged tiles, 3 whole rows, 4 pipelined whole rows")
     return p.parse_args()
 
 

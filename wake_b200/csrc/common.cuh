@@ -10,7 +10,8 @@
 // resident per SM. Two nodes per thread: 64 x 8 gives D3Q19 / D3Q27 128 registers (16 warps per SM), which their 38 / 54
 // loads in flight need without spills. Sphere channel FP32 256x128x128, 160^3, 48^3: 108.5, 108.9, 6.8 us a step; at
 // 96 registers (20 warps) 119.1, 120.1, 9.0. D2Q9 carries half the values: 64 registers and 32 warps (2048x1024:
-// 22.0 us, 25.1 with 96 registers); 96 where a batch's arguments have to be read (60 channels: 56.2 -> 52.2 us).
+// 22.0 us, 25.1 with 96 registers); 80 where a batch's arguments have to be read (60 channels: 52.0 us a step, 56.7
+// with 96 registers, 53.5 with 72).
 #ifndef WK_FAST_MAX_THREADS
 #define WK_FAST_MAX_THREADS 64
 #endif

@@ -1,0 +1,96 @@
+"""Steps over geometry, models and options that the scenario tests do not combine, against the oracle.
+
+Tolerances are those of the other oracle comparisons: velocity within twice an FP32 CPU implementation's error against
+FP64 (or 1e-5), density 1e-5, force history 1e-4.
+"""
+import numpy as np
+import pytest
+
+from conftest import rel_l2, vel_rel_l2
+from test_gpu_grid import FORCE_TOL, RHO_TOL, U_TOL
+
+pytestmark = pytest.mark.gpu
+
+wb = pytest.importorskip("wake_b200")
+import oracle  # noqa: E402
+
+STEPS = 20
+TAU = 0.56
+GRIDS = {9: wb.LatticeGrid2D, 19: wb.LatticeGrid3D, 27: wb.LatticeGrid3DQ27}
+
+
+def _waves(q, nx, ny, nz):
+    """Density and velocity of a few long waves, every component non-zero, as float32 arrays."""
+    z, y, x = np.meshgrid(np.arange(nz), np.arange(ny), np.arange(nx), indexing="ij")
+    a, b, c = (2.0 * np.pi * v / n for v, n in ((x, nx), (y, ny), (z, nz)))
+    u = (0.04 + 0.02 * np.sin(a + b + 0.3), 0.02 * np.cos(a - c) + 0.01 * np.sin(b), 0.015 * np.sin(c + a + 1.0))
+    rho = 1.0 + 0.01 * np.sin(a + 2.0 * b)
+    out = [np.ascontiguousarray(v, np.float32).ravel() for v in (rho, *u)]
+    if q == 9:
+        out[3] = np.zeros_like(out[3])
+    return out
+
+
+def _step_both(q, size, types, collision, les=False, force=(0.0, 0.0, 0.0), wall=None, periodic=(False, False), links=None,
+               mem=None, tau=TAU, steps=STEPS):
+    """(grid, oracle FP32, oracle FP64, its FP32 force history) after the same steps from the same populations.
+    wall: velocity of the MOVING_WALL cells; links: (node, direction, delta, velocity)."""
+    nx, ny, nz = size
+    types = np.ascontiguousarray(types, np.uint8).ravel()
+    f0 = oracle.equilibrium(q, *_waves(q, nx, ny, nz), prec=32).astype(np.float32)
+    g = GRIDS[q](nx, ny, tau) if q == 9 else GRIDS[q](nx, ny, nz, tau)
+    if wall is not None:
+        wb.check(wb.lib.wake_grid_set_moving_wall(g.handle, *wall))
+    g.set_cell_types(types)
+    if q != 9:
+        g.set_periodic_axes(*periodic)
+    if links is not None:
+        g.set_curved_links(*links)
+    g.set_populations(f0)
+    if mem is not None:
+        g.enable_forces(*mem)
+    gz = {} if q == 9 else {"gz": force[2]}
+    g.step(collision, gx=force[0], gy=force[1], use_les=les, smag_const=0.17, n=steps, **gz)
+    g.synchronize()
+    out = [g]
+    for prec in (32, 64):
+        o = oracle.OracleGrid(q, nx, ny, nz, prec)
+        kw = {} if wall is None else {"u_wall": wall}
+        if mem is not None:
+            kw.update(mem=1, center=mem[:3], r_max=mem[3])
+        o.configure(collision=collision, tau=tau, les=int(les), cs_smag=0.17, g=force, periodic_y=int(periodic[0]),
+                    periodic_z=int(periodic[1]), **kw)
+        o.set_cell_types(types)
+        o.set_state(f0)
+        if links is not None:
+            o.set_links(*links)
+        hist = o.step(steps, forces=mem is not None)
+        out.append(o)
+        if prec == 32:
+            h32 = hist
+    return (*out, h32)
+
+
+def _check(q, *args, **kw):
+    g, o32, o64, h32 = _step_both(q, *args, **kw)
+    keys = ("ux", "uy") if q == 9 else ("ux", "uy", "uz")
+    m, m32, m64 = g.macro(), o32.macro(), o64.macro()
+    e64, e_o64 = vel_rel_l2(m, m64, keys), vel_rel_l2(m32, m64, keys)
+    print(f"[D?Q{q}] u vs FP64 {e64:.2e} (oracle-fp32 {e_o64:.2e}), rho vs oracle-fp32 {rel_l2(m['rho'], m32['rho']):.2e}")
+    assert e64 <= max(U_TOL, 2.0 * e_o64)
+    assert rel_l2(m["rho"], m32["rho"]) <= RHO_TOL
+    if kw.get("mem") is not None:
+        hist = g.force_history()
+        assert hist.shape[0] == STEPS and np.any(h32 != 0.0) and rel_l2(hist, h32) <= FORCE_TOL
+
+
+@pytest.mark.parametrize("collision", [wb.BGK, wb.TRT, wb.MRT])
+@pytest.mark.parametrize("q,size,solid", [(9, (72, 64, 1), (68, 63, 0)), (19, (80, 16, 12), (72, 15, 11)),
+                                          (27, (80, 16, 12), (72, 15, 11))])
+def test_pure_run_ends_within_the_last_inner_row(q, size, solid, collision):
+    """A cell shorter than 64 nodes at the end of the last rows whose pulls stay inside, in a lattice whose node count
+    leaves no padding behind the planes."""
+    nx, ny, nz = size
+    types = np.zeros((nz, ny, nx), np.uint8)
+    types[solid[2], solid[1], solid[0]] = wb.SOLID
+    _check(q, size, types, collision)

@@ -72,18 +72,20 @@ __device__ __forceinline__ PullOffsets pull_offsets(const Geo& g, unsigned i) {
     o.yp = y == ny - 1 ? (1 - ny) * nx : nx;
     return o;
 }
-// How a pure cell gathers. INSIDE: no node pulls across a face, so direction q's source is the node's index
-// minus one constant and its address one addition to a per-launch base. ROW_ENDS: as INSIDE in y and z,
-// but a row ends in the cell, whose end nodes wrap in x. FACES: a y or z face is in reach.
+// How a pure cell gathers. INSIDE: a whole cell of which no node pulls across a face, so direction q's source is the
+// node's index minus one constant and its address one addition to a per-launch base, which cell_pairs takes for a lane's
+// second node too without asking whether it exists (a shorter cell near the lattice's end would read past the
+// plane). ROW_ENDS: as INSIDE in y and z, but a row ends in the cell, whose end nodes wrap in x, or the cell is
+// shorter. FACES: a y or z face is in reach.
 enum CellGather { INSIDE, ROW_ENDS, FACES };
 template <int Q>
-__device__ __forceinline__ CellGather cell_gather(const Geo& g, unsigned i0, int count) {
+__host__ __device__ __forceinline__ CellGather cell_gather(const Geo& g, unsigned i0, int count) {
     const unsigned nx = g.nx, last = i0 + count - 1, r0 = g.by_nx.quot(i0), r1 = g.by_nx.quot(last);
     const unsigned z = Lat<Q>::D == 3 ? g.by_ny.quot(r0) : 0u, y0 = r0 - z * g.ny, y1 = y0 + (r1 - r0);
     const bool in_y = y0 > 0u && y1 < static_cast<unsigned>(g.ny) - 1u;
     const bool in_z = Lat<Q>::D == 2 || (z > 0u && z < static_cast<unsigned>(g.nz) - 1u);
     if (!in_y || !in_z) return FACES;
-    return r0 == r1 && i0 != r0 * nx && last != r0 * nx + nx - 1u ? INSIDE : ROW_ENDS;
+    return count == CELL && r0 == r1 && i0 != r0 * nx && last != r0 * nx + nx - 1u ? INSIDE : ROW_ENDS;
 }
 template <int Q>
 __device__ __forceinline__ int pull_offset(const PullOffsets& o, int q) {

@@ -34,7 +34,9 @@ struct FastDiv {
         while ((1ull << l) < d) ++l;
         return {static_cast<unsigned>(((1ull << (31 + l)) + d - 1) / d), l - 1u};
     }
-    __device__ __forceinline__ unsigned quot(unsigned n) const { return m ? __umulhi(n, m) >> s : n; }
+    __host__ __device__ __forceinline__ unsigned quot(unsigned n) const {
+        return m ? static_cast<unsigned>((static_cast<unsigned long long>(n) * m) >> 32) >> s : n;
+    }
 };
 
 struct Geo {

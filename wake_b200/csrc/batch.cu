@@ -194,8 +194,11 @@ int batch_prepare(wake_batch* b) {
         if (m.g->collision != g0->collision || m.g->les != g0->les)
             return set_error(WAKE_ERR_INVALID, "wake_batch: members differ in collision model or LES switch");
     }
-    b->coll = g0->collision;
-    b->les = g0->les;
+    if (b->coll != g0->collision || b->les != g0->les) {
+        b->coll = g0->collision;
+        b->les = g0->les;
+        ++b->shape;  // a captured graph holds the other model's kernel
+    }
     for (const auto& m : b->members) {
         const int r = grid_prepare(m.g);
         if (r) return r;

@@ -37,3 +37,34 @@ def test_graph_follows_a_change_of_model(q, storage):
                 alone.step(collision, use_les=les, smag_const=0.17, n=8)
             assert np.array_equal(g.f_src_data(), alone.f_src_data())
             assert np.array_equal(g.force_history(), alone.force_history())
+
+
+def test_graph_follows_a_change_of_a_member_beyond_32_bit_offsets():
+    """A member of 2^32 or more values steps by its own launches, whose arguments a graph holds by value."""
+    nx = ny = 21846
+    assert 9 * nx * ny >= 1 << 32
+
+    def flow():
+        g = wb.LatticeGrid2D(nx, ny, 0.6, storage="f16")
+        wb.check(wb.lib.wake_grid_initialize_noise(g.handle, 1.0, 0.04, 0.0, 0.0, 0.02, 7, 0))
+        return g
+
+    with Batch(9, "f16") as batch:
+        g = flow()
+        batch.add(g, wb.BGK)
+        batch.use_graph(2)
+        batch.step(2)
+        g.set_relaxation_time(0.9)
+        batch.step(2)
+        batch.synchronize()
+        got = g._diag()
+        batch.remove(g)
+        g.close()
+    alone = flow()
+    alone.step(wb.BGK, n=2)
+    alone.set_relaxation_time(0.9)
+    alone.step(wb.BGK, n=2)
+    want = alone._diag()
+    alone.close()
+    wb.lib.wake_gpu_cache_trim()
+    assert got == want

@@ -152,13 +152,19 @@ int build_tables(wake_batch* b) {
     if (dom.size() == b->up_dom.size() &&
         (dom.empty() || std::memcmp(dom.data(), b->up_dom.data(), sizeof(BatchDom) * n) == 0))
         return WAKE_OK;
+    // a captured graph keeps launch shapes and table addresses, not the table contents; only the launches of a member
+    // that is stepped by itself hold its arguments by value
+    for (std::size_t i = 0; i < n; ++i)
+        if (dom[i].alone && i < b->up_dom.size() && std::memcmp(&dom[i], &b->up_dom[i], sizeof(BatchDom)) != 0) {
+            ++b->shape;
+            break;
+        }
     WK_CUDA(cudaStreamSynchronize(b->stream));  // queued steps may still read the old table
     const void* old_dom = b->d_dom.p;
     WK_CUDA(b->d_dom.grow(sizeof(BatchDom) * std::max<std::size_t>(1, n)));
     if (n) WK_CUDA(cudaMemcpyAsync(b->d_dom.p, dom.data(), sizeof(BatchDom) * n, cudaMemcpyHostToDevice, b->stream));
     WK_CUDA(cudaStreamSynchronize(b->stream));
     b->up_dom = std::move(dom);
-    // a captured graph keeps launch shapes and table addresses, not the table contents
     if (old_dom != b->d_dom.p) ++b->shape;
     return WAKE_OK;
 }

@@ -52,6 +52,7 @@ def test_graph_follows_a_change_of_a_member_beyond_32_bit_offsets():
     with Batch(9, "f16") as batch:
         g = flow()
         batch.add(g, wb.BGK)
+        assert batch.info()["launches_per_step"] == 1
         batch.use_graph(2)
         batch.step(2)
         g.set_relaxation_time(0.9)

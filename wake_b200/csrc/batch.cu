@@ -403,8 +403,10 @@ int wake_batch_info(wake_batch* b, long long* nodes, int* bulk_rows, int* genera
     if (nodes) *nodes = nn;
     if (bulk_rows) *bulk_rows = b->n_pure;
     if (general_rows) *general_rows = b->n_listed;
-    if (launches_per_step)
+    if (launches_per_step) {
         *launches_per_step = b->n_pure + b->n_listed > 0 ? 1 : 0;
+        for (const BatchDom& d : b->up_dom) *launches_per_step += d.alone;
+    }
     return WAKE_OK;
 }
 

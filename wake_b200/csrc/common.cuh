@@ -30,10 +30,14 @@ namespace wk {
 int set_error(int code, const std::string& msg);
 void clear_error();
 
+// Return with a failed call's error, and take it from the runtime: the check of the next launch would report it again.
 #define WK_CUDA(call)                                                                                      \
     do {                                                                                                   \
         cudaError_t e_ = (call);                                                                           \
-        if (e_ != cudaSuccess) return ::wk::set_error(-2, std::string(#call) + ": " + cudaGetErrorString(e_)); \
+        if (e_ != cudaSuccess) {                                                                           \
+            (void)cudaGetLastError();                                                                      \
+            return ::wk::set_error(-2, std::string(#call) + ": " + cudaGetErrorString(e_));                \
+        }                                                                                                  \
     } while (0)
 
 // Device blocks are taken from, and may be handed back to, a process-wide cache

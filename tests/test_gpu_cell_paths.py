@@ -94,3 +94,27 @@ def test_pure_run_ends_within_the_last_inner_row(q, size, solid, collision):
     types = np.zeros((nz, ny, nx), np.uint8)
     types[solid[2], solid[1], solid[0]] = wb.SOLID
     _check(q, size, types, collision)
+
+
+def test_moments_into_a_buffer_that_is_too_short_are_refused():
+    """A device buffer whose allocation ends before the field does: an error from the host, as from a copy to it."""
+    import ctypes
+
+    import torch
+
+    torch.cuda.synchronize()
+    g = wb.LatticeGrid2D(65, 33, TAU)
+    g.step(wb.TRT, n=2)
+    cuda = ctypes.CDLL("libcuda.so.1")
+    p = ctypes.c_uint64()
+    assert cuda.cuMemAlloc_v2(ctypes.byref(p), ctypes.c_size_t(4096)) == 0  # 65 x 33 floats take 8,580 B
+    try:
+        with pytest.raises(RuntimeError):
+            wb.check(wb.lib.wake_grid_get_macroscopic(g.handle, None, ctypes.c_void_p(p.value), None, None, None))
+    finally:
+        assert cuda.cuMemFree_v2(p) == 0
+    wb.lib.wake_gpu_clear_error()
+    whole = torch.zeros(65 * 33, dtype=torch.float32, device="cuda")
+    torch.cuda.synchronize()
+    g.macroscopic_into(ux=whole)
+    assert np.array_equal(whole.cpu().numpy(), g.macro()["ux"])

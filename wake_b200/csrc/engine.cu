@@ -14,6 +14,8 @@
 #include <string>
 #include <vector>
 
+#include <cuda.h>
+
 #include "analytics.cuh"
 #include "engine.cuh"
 
@@ -1747,6 +1749,25 @@ int wake_grid_get_populations(wake_grid* g, float* f) {
     return WAKE_OK;
 }
 
+// Bytes from device pointer p to the end of its allocation; 0 where the driver does not say.
+static std::size_t allocated_from(const void* p) {
+    static const auto range = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult found{};
+        if (cudaGetDriverEntryPointByVersion("cuMemGetAddressRange", &f, 12000, cudaEnableDefault, &found) != cudaSuccess ||
+            found != cudaDriverEntryPointSuccess) {
+            (void)cudaGetLastError();
+            f = nullptr;
+        }
+        return reinterpret_cast<decltype(&cuMemGetAddressRange)>(f);
+    }();
+    CUdeviceptr base = 0;
+    std::size_t size = 0;
+    const auto at = reinterpret_cast<CUdeviceptr>(p);
+    if (!range || range(&base, &size, at) != CUDA_SUCCESS) return 0;
+    return static_cast<std::size_t>(base + size - at);
+}
+
 int wake_grid_get_macroscopic(wake_grid* g, float* rho, float* ux, float* uy, float* uz, float* speed) {
     if (!valid_grid(g)) return WAKE_ERR_INVALID;
     int r = ensure_macro(g);
@@ -1756,14 +1777,16 @@ int wake_grid_get_macroscopic(wake_grid* g, float* rho, float* ux, float* uy, fl
     Out o = scratch_out(g, false, true);
     float** const field[5] = {&o.rho, &o.ux, &o.uy, &o.uz, &o.speed};
     float* copy[5] = {};
-    // Straight into the caller's memory where it is this device's, holds aligned floats and overlaps nothing that the
+    // Straight into the caller's memory where it is this device's, holds aligned floats, lies in one allocation (a copy
+    // to less memory than that is refused, a kernel would write past it) and overlaps nothing that the
     // kernel reads or writes beside it, by way of the scratch otherwise: a copy per field costs 40 B a node more
     // and, on a small lattice, its own launch (a D2Q9 65x33 step and its four fields: 31.9 -> 19.3 us).
     cudaPointerAttributes own{};
     WK_CUDA(cudaPointerGetAttributes(&own, g->A.p));
     const auto here = [&](const void* p) {
         cudaPointerAttributes a{};
-        if (cudaPointerGetAttributes(&a, p) == cudaSuccess) return a.type == cudaMemoryTypeDevice && a.device == own.device;
+        if (cudaPointerGetAttributes(&a, p) == cudaSuccess)
+            return a.type == cudaMemoryTypeDevice && a.device == own.device && allocated_from(p) >= b;
         (void)cudaGetLastError();
         return false;
     };

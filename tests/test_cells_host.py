@@ -1,4 +1,4 @@
-"""Index arithmetic of the cell gathers, run on the host."""
+"""Arithmetic of the step kernels that runs on the host too: the cells' indexes, the division of the Zou-He faces."""
 import shutil
 import subprocess
 from pathlib import Path
@@ -8,16 +8,20 @@ import pytest
 ROOT = Path(__file__).resolve().parents[1]
 
 
-@pytest.fixture(scope="module")
-def reach(tmp_path_factory):
+def _compile(source, folder):
     nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
     if not Path(nvcc).exists():
         pytest.skip("no nvcc")
-    exe = tmp_path_factory.mktemp("cells") / "cells_reach"
-    subprocess.run([nvcc, "-std=c++17", "-O1", "--expt-relaxed-constexpr", "-gencode", "arch=compute_100a,code=sm_100a",
-                    f"-I{ROOT / 'wake_b200' / 'csrc'}", f"-I{ROOT / 'include'}", str(ROOT / "tests" / "cells_reach.cu"),
+    exe = folder / source
+    subprocess.run([nvcc, "-std=c++17", "-O2", "--expt-relaxed-constexpr", "-gencode", "arch=compute_100a,code=sm_100a",
+                    f"-I{ROOT / 'wake_b200' / 'csrc'}", f"-I{ROOT / 'include'}", str(ROOT / "tests" / f"{source}.cu"),
                     "-o", str(exe)], check=True)
     return exe
+
+
+@pytest.fixture(scope="module")
+def reach(tmp_path_factory):
+    return _compile("cells_reach", tmp_path_factory.mktemp("cells"))
 
 
 # Node counts that are a multiple of the plane's padding (64), where the last plane ends with its last node, rows
@@ -27,4 +31,10 @@ def reach(tmp_path_factory):
                                         (27, 72, 8, 8)])
 def test_inside_cells_read_their_plane_only(reach, q, nx, ny, nz):
     r = subprocess.run([str(reach), str(q), str(nx), str(ny), str(nz)], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout
+
+
+def test_division_by_a_constant(tmp_path):
+    """By 3 and 6 over every 251st float (every 7th of the smallest), the zeros, the largest, infinity and NaN."""
+    r = subprocess.run([str(_compile("by_const", tmp_path))], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stdout

@@ -755,14 +755,18 @@ __device__ __forceinline__ void collide(float* f, float rho, const float u[3], c
 }
 
 // ---------------------------------------------------------------- Zou-He
-// x / D correctly rounded, in three instructions: the quotient estimate x RN(1/D), its exact remainder and the correction
-// (Markstein, "Computation of elementary functions on the IBM RISC System/6000 processor", 1990). A division takes about
-// ten, and the D3Q19 faces divide eight times.
+// x / D as the division gives it, D = 3 or 6: the quotient estimate q = x RN(1/D), its exact remainder and the
+// correction (Markstein, "Computation of elementary functions on the IBM RISC System/6000 processor", 1990). A remainder of
+// zero leaves q (exact, and -0 keeps its sign), as does that of an infinity, which is no number. Only where D = 6 and
+// a subnormal quotient lies midway between two does the correction decide the tie (2^-149 off at most). A division takes
+// about ten instructions, and the D3Q19 faces divide eight times: with divisions an 81^3 sphere job of 200 steps takes
+// 4.73 ms instead of 4.22, the FP32 256x128x128 channel 124 us a step instead of 121.
 template <int D>
-__device__ __forceinline__ float by_const(float x) {
+__host__ __device__ __forceinline__ float by_const(float x) {
     constexpr float y = 1.0f / D;
-    const float q = __fmul_rn(x, y);
-    return __fmaf_rn(__fmaf_rn(-float(D), q, x), y, q);
+    const float q = x * y, r = fmaf(-float(D), q, x);
+    if (!(fabsf(r) > 0.0f)) return q;
+    return fmaf(r, y, q);
 }
 
 // 2D: d2q9_boundaries.ispc:43-121. 3D: Hecht & Harting (2010) on-site velocity

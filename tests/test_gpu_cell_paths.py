@@ -143,3 +143,33 @@ def test_outlet_face_keeps_an_infinite_correction():
     want = o.f()
     assert np.count_nonzero(np.isneginf(want)) == 5 * ny * nz  # directions 2, 8, 10, 12, 14 of the face
     assert np.array_equal(np.isneginf(got), np.isneginf(want)) and np.array_equal(np.isnan(got), np.isnan(want))
+
+
+def test_forces_of_a_callers_graph_between_steps_of_another_kernel():
+    """Replays of a graph the caller captured with one kernel and steps with another leave one history in order."""
+    import torch
+
+    from wake_b200 import workloads as W
+
+    case = W.sphere_channel(64, 16, 16, 4.0, (20.0, 8.0, 8.0), tau=0.55, collision=wb.TRT)
+    model = dict(use_les=case.les, smag_const=case.cs_smag)
+    g, alone = W.build_grid(case, storage="f16"), W.build_grid(case, storage="f16")
+    stream = torch.cuda.Stream()
+    g.set_stream(stream.cuda_stream)
+    g.step(case.collision, n=2, **model)
+    assert wb.lib.wake_grid_get_kernel(g.handle) == 4
+    g.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        g.step(case.collision, n=2, **model)
+    with torch.cuda.stream(stream):
+        graph.replay()
+        for _ in range(3):
+            wb.check(wb.lib.wake_grid_set_kernel(g.handle, 1))
+            g.step(case.collision, n=2, **model)
+            graph.replay()
+    got = g.force_history()
+    alone.step(case.collision, n=16, **model)
+    want = alone.force_history()
+    assert want.shape[0] == 16 and np.all(np.any(want != 0.0, axis=1))
+    assert np.array_equal(got, want)

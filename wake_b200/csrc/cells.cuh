@@ -201,11 +201,10 @@ __device__ __forceinline__ void curved_links(const typename Codec<S>::T* fin, lo
 // of the slots and a fixed tree, whatever the launch, so the force is reproducible bit for bit.
 __device__ __forceinline__ void mem_sum(const MemCfg& M) {
     const int lane = threadIdx.x & 31;
-    const unsigned pending = *M.pending;
-    if (pending == 0u) return;
-    const int slots = M.slots;
-    const double* part = M.contrib + (pending - 1u) * M.stride;
-    const unsigned step = *M.hist_step;
+    const double* part = M.left->part;
+    if (!part) return;
+    const int slots = M.left->slots;
+    const unsigned step = M.left->steps;
 #pragma unroll 1
     for (int c = 0; c < 3; ++c) {  // one component at a time: this rare path must not set the kernel's registers
         double s[8];
@@ -225,14 +224,17 @@ __device__ __forceinline__ void mem_sum(const MemCfg& M) {
         if (lane == 0) M.hist[3 * static_cast<long long>(step % static_cast<unsigned>(M.hist_cap)) + c] = s[0];
     }
     __syncwarp();
-    if (lane == 0) *M.hist_step = step + 1u;
+    if (lane == 0) M.left->steps = step + 1u;
 }
 
 // The same at the start of a step that reads buffer `cur`, which leaves its own partial sums outstanding.
 __device__ __forceinline__ void mem_sum_step(const MemCfg& M, int cur) {
     mem_sum(M);
     __syncwarp();
-    if ((threadIdx.x & 31) == 0) *M.pending = 1u + static_cast<unsigned>(cur);
+    if ((threadIdx.x & 31) == 0) {
+        M.left->part = M.contrib + cur * M.stride;
+        M.left->slots = M.slots;
+    }
 }
 
 // The momentum exchange of a cell's (half cell's) nodes, in all lanes, to its slot.

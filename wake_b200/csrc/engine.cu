@@ -234,7 +234,7 @@ __global__ void k_diag_partials(const float* __restrict__ rho, const float* __re
 __global__ void k_mem_flush(const MemCfg mem) {
     mem_sum(mem);
     __syncwarp();
-    if (threadIdx.x == 0) *mem.pending = 0u;
+    if (threadIdx.x == 0) mem.left->part = nullptr;
 }
 
 // ---------------------------------------------------------------- device initialisation
@@ -448,8 +448,8 @@ int rebuild_flags(wake_grid* g) {
 
 // Append the last step's outstanding force.
 int flush_force(wake_grid* g) {
-    if (!g->mem_on || g->mem_list == 0 || !(g->mem_left || g->mem_captured)) return WAKE_OK;
-    const StepArgs a = wk::grid_step_args(g, g->mem_list == 2);
+    if (!g->mem_on || !(g->mem_left || g->mem_captured)) return WAKE_OK;
+    const StepArgs a = wk::grid_step_args(g);
     k_mem_flush<<<1, 32, 0, g->stream>>>(a.mem);
     WK_CUDA(cudaGetLastError());
     g->mem_left = false;
@@ -850,7 +850,6 @@ int prepare_state(wake_grid* g) {
 int prepare(wake_grid* g) {
     int r = prepare_state(g);
     if (!r) r = ensure_lists(g);
-    if (!r && g->mem_list != 0 && g->mem_list != (g->by_rows() ? 2 : 1)) r = flush_force(g);  // the other list's slots
     return r;
 }
 
@@ -938,7 +937,7 @@ int do_steps(wake_grid* g, int n) {
         for (int c = 0; c < 3; ++c) g->last_step_g[c] = g->phys.g[c];
         ++g->k;
     }
-    if (n > 0 && g->mem_on) wk::grid_force_left(g, by_rows);
+    if (n > 0 && g->mem_on) wk::grid_force_left(g);
     return WAKE_OK;
 }
 
@@ -951,7 +950,6 @@ int grid_prepare(wake_grid* g) {
     int r = prepare_state(g);
     if (!r) r = ensure_cells(g);
     if (!r) r = ensure_units(g, g->cells);
-    if (!r && g->mem_list == 2) r = flush_force(g);
     return r;
 }
 
@@ -981,8 +979,7 @@ StepArgs grid_step_args(const wake_grid* g, bool rest) {
         a.mem.slots = L.slots;
         a.mem.contrib = L.contrib.as<double>();
         a.mem.stride = L.stride;
-        a.mem.pending = g->d_counters.as<unsigned>();
-        a.mem.hist_step = g->d_counters.as<unsigned>() + 1;
+        a.mem.left = g->d_left.as<wk::MemLeft>();
         a.mem.hist = g->d_hist.as<double>();
         a.mem.hist_cap = g->hist_cap;
     }
@@ -1018,8 +1015,7 @@ void grid_step_buffers(wake_grid* g, int cur, StepArgs& a) {
     }
 }
 
-void grid_force_left(wake_grid* g, bool rest) {
-    g->mem_list = rest ? 2 : 1;
+void grid_force_left(wake_grid* g) {
     g->mem_left = true;
     ++g->mem_issued;
     cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
@@ -1028,7 +1024,7 @@ void grid_force_left(wake_grid* g, bool rest) {
 
 void grid_advanced(wake_grid* g, int n) {
     if (n <= 0) return;
-    if (g->mem_on) grid_force_left(g, false);
+    if (g->mem_on) grid_force_left(g);
     g->cur ^= (n & 1);
     g->k += n;
     g->mf_valid = false;
@@ -1577,9 +1573,9 @@ int wake_grid_enable_forces(wake_grid* g, float cx, float cy, float cz, float r_
     g->hist_seen = 0;
     g->seen_at = ~0ull;
     WK_CUDA(g->d_hist.ensure(sizeof(double) * 3 * history_capacity));
-    WK_CUDA(g->d_counters.ensure(sizeof(unsigned) * 2));
-    WK_CUDA(cudaMemsetAsync(g->d_counters.p, 0, sizeof(unsigned) * 2, g->stream));
-    g->mem_list = 0;
+    WK_CUDA(g->d_left.ensure(sizeof(wk::MemLeft)));
+    WK_CUDA(cudaMemsetAsync(g->d_left.p, 0, sizeof(wk::MemLeft), g->stream));
+    g->mem_left = false;
     WK_CUDA(cudaMemsetAsync(g->d_hist.p, 0, sizeof(double) * 3 * history_capacity, g->stream));
     // the flags carry the momentum-exchange bit; a pending geometry change
     // is applied (with its state resync) by the next step instead
@@ -1604,11 +1600,11 @@ int wake_grid_disable_forces(wake_grid* g) {
 
 long long wake_grid_force_count(wake_grid* g) {
     if (!valid_grid(g) || !g->mem_on) return 0;
-    unsigned c[2] = {0, 0};
-    if (cudaMemcpyAsync(c, g->d_counters.p, sizeof(c), cudaMemcpyDeviceToHost, g->stream) != cudaSuccess ||
+    wk::MemLeft left{};
+    if (cudaMemcpyAsync(&left, g->d_left.p, sizeof(left), cudaMemcpyDeviceToHost, g->stream) != cudaSuccess ||
         cudaStreamSynchronize(g->stream) != cudaSuccess)
         return set_error(WAKE_ERR_CUDA, "wake_grid_force_count: copy failed");
-    g->hist_seen = static_cast<long long>(c[1]) + (c[0] != 0u ? 1 : 0);  // with the outstanding one
+    g->hist_seen = static_cast<long long>(left.steps) + (left.part ? 1 : 0);  // with the outstanding one
     g->seen_at = g->mem_issued;
     return g->hist_seen;
 }
@@ -1658,7 +1654,6 @@ static int capture_graph(wake_grid* g) {
     g->graph_ok = false;
     const int cur0 = g->cur;
     const long long k0 = g->k;
-    const int list0 = g->mem_list;
     const bool left0 = g->mem_left, captured0 = g->mem_captured;
     cudaGraph_t graph = nullptr;
     WK_CUDA(cudaStreamBeginCapture(g->stream, cudaStreamCaptureModeThreadLocal));
@@ -1666,7 +1661,6 @@ static int capture_graph(wake_grid* g) {
     cudaError_t e = cudaStreamEndCapture(g->stream, &graph);
     g->cur = cur0;
     g->k = k0;
-    g->mem_list = list0;
     g->mem_left = left0;
     g->mem_captured = captured0;
     if (r) {
@@ -1701,7 +1695,7 @@ int wake_grid_step(wake_grid* g, int n, float gx, float gy, float gz) {
             g->k += gs;
             g->mf_valid = false;
             for (int c = 0; c < 3; ++c) g->last_step_g[c] = g->phys.g[c];
-            if (g->mem_on) wk::grid_force_left(g, g->by_rows());
+            if (g->mem_on) wk::grid_force_left(g);
             done += gs;
         }
     }
@@ -1978,7 +1972,7 @@ int wake_grid_info(wake_grid* g, int* q, int* nx, int* ny, int* nz, int* storage
 long long wake_grid_device_bytes(wake_grid* g) {
     if (!valid_grid(g)) return WAKE_ERR_INVALID;
     const DevMem* all[] = {&g->A, &g->B, &g->d_types, &g->d_flags, &g->d_status, &g->d_nodestart, &g->d_link_node,
-                           &g->d_link_rec, &g->d_link_mom, &g->d_counters, &g->d_hist, &g->d_kind, &g->d_seg, &g->d_row_kind,
+                           &g->d_link_rec, &g->d_link_mom, &g->d_left, &g->d_hist, &g->d_kind, &g->d_seg, &g->d_row_kind,
                            &g->d_row_list, &g->d_tiles, &g->m_f, &g->m_rho, &g->m_ux, &g->m_uy, &g->m_uz, &g->m_speed,
                            &g->m_diag, &g->TA, &g->TB, &g->m_t, &g->m_an};
     long long sum = static_cast<long long>(g->cells.bytes() + g->rest.bytes());

@@ -119,13 +119,12 @@ struct wake_grid {
 
     int mem_on = 0, hist_cap = 0;
     float center[3] = {0.f, 0.f, 0.f}, rmax = 0.f;
-    DevMem d_counters, d_hist;  // counters: [0] outstanding force (MemCfg::pending), [1] history entries written
+    DevMem d_left, d_hist;  // MemLeft, history
     // the history's length as read last, the value of mem_issued then (~0: never); calls that issued steps with forces on
     long long hist_seen = 0;
     unsigned long long seen_at = ~0ull, mem_issued = 0;
-    // whose slots the last step left its force in (0 none, 1 `cells`, 2 `rest`), whether it may still be outstanding, and
-    // whether steps were captured into a caller's graph, whose replays leave forces unseen by the host
-    int mem_list = 0;
+    // whether the last step's force may still be outstanding, and whether steps were captured into a caller's graph, whose
+    // replays leave forces unseen by the host
     bool mem_left = false, mem_captured = false;
 
     // k_step_cells: what the linear cells and the segments are, and the cells that are listed
@@ -201,7 +200,7 @@ struct wake_grid {
         if (side) idle = idle && cudaStreamSynchronize(side) == cudaSuccess;
         if (idle) {
             DevMem* all[] = {&A, &B, &d_types, &d_flags, &d_status, &d_nodestart, &d_link_node, &d_link_rec,
-                             &d_link_mom, &d_counters, &d_hist, &d_kind, &d_seg, &d_row_kind, &d_row_list, &d_tiles, &m_f,
+                             &d_link_mom, &d_left, &d_hist, &d_kind, &d_seg, &d_row_kind, &d_row_list, &d_tiles, &m_f,
                              &m_rho, &m_ux, &m_uy, &m_uz, &m_speed, &m_diag, &TA, &TB, &m_t, &m_an};
             cells.release();
             rest.release();
@@ -287,8 +286,8 @@ StepArgs grid_step_args(const wake_grid* g, bool rest = false);
 bool fits_l2(long long bytes);
 // Its buffers: the state in buf(cur), the step's output in the other one.
 void grid_step_buffers(wake_grid* g, int cur, StepArgs& a);
-// The last step left its force in the slots of `rest` (else `cells`).
-void grid_force_left(wake_grid* g, bool rest);
+// The last step left its force outstanding.
+void grid_force_left(wake_grid* g);
 // Bookkeeping after n steps run outside wake_grid_step (by a batch).
 void grid_advanced(wake_grid* g, int n);
 // Error status word of the lattice: WAKE_OK or WAKE_ERR_NUMERIC (synchronizes its stream).

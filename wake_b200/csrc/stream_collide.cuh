@@ -62,19 +62,25 @@ struct Links {
     int count;
 };
 
+struct MemLeft {                  // in device memory: what the steps so far left of the forces
+    const double* part;           // the last step's force, `slots` partial sums, while it is not in the history yet
+    int slots;
+    unsigned steps;               // number of entries written to the history
+};
+
 struct MemCfg {                   // momentum-exchange monitor
     int enabled;
     float center[3];
     // Every unit of the listed cells with momentum-exchange links owns one slot of `contrib` (slot[2 * entry + half];
     // a whole cell's is slot[2 * entry]), numbered in node order, in the half of `contrib` of the buffer the step
     // reads (stride doubles apart). The next launch sums them in slot order: the force is reproducible bit for bit.
-    // Any list of cells that holds these nodes gives the same sums.
+    // Any list of cells that holds these nodes gives the same sums, and `left` says where they are: a graph that a
+    // caller captured may follow steps over another list.
     const int* slot;
     int slots;
     double* contrib;              // [2][slots][3]
     long long stride;
-    unsigned* pending;            // 0, or 1 + the half of `contrib` that is not summed yet
-    unsigned* hist_step;          // number of entries written so far
+    MemLeft* left;
     double* hist;                 // [hist_cap][3]: (Fx, Fy, Tz) in 2D, (Fx, Fy, Fz) in 3D
     int hist_cap;
 };

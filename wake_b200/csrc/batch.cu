@@ -178,7 +178,7 @@ int batch_steps(wake_batch* b, int n) {
         a.pure = b->d_pure.as<uint2>();
         a.npure = static_cast<unsigned>(b->n_pure);
         a.parity = b->parity;
-        a.evict_first = fits_l2(b->state_bytes);
+        a.evict_first = fits_l2(b->members[0].g, b->state_bytes);
         WK_CUDA(launch_batch_any(b->Q, b->coll, b->storage, b->les != 0, a, b->thermal, b->tpb, b->stream));
         for (std::size_t i = 0; i < b->up_dom.size(); ++i) {
             if (!b->up_dom[i].alone) continue;

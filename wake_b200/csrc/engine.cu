@@ -955,14 +955,8 @@ int grid_prepare(wake_grid* g) {
 
 // Whether a state buffer of that many bytes is read evict-first (read_policy): up to three quarters of the L2, above
 // which it no longer helps (D3Q19 107 MB, 131 MB) and a batch of 108 MB lost 3 %.
-bool fits_l2(long long bytes) {
-    static int l2 = 0;
-    if (l2 == 0) {
-        int dev = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev) != cudaSuccess)
-            l2 = 126 << 20;
-    }
-    return bytes <= l2 / 4 * 3ll;
+bool fits_l2(const wake_grid* g, long long bytes) {
+    return bytes <= g->l2_bytes / 4 * 3ll;
 }
 
 StepArgs grid_step_args(const wake_grid* g, bool rest) {
@@ -984,7 +978,7 @@ StepArgs grid_step_args(const wake_grid* g, bool rest) {
         a.mem.hist_cap = g->hist_cap;
     }
     a.phys = g->phys;
-    a.evict_first = fits_l2(static_cast<long long>(g->elem) * g->Q * g->pitch);
+    a.evict_first = fits_l2(g, static_cast<long long>(g->elem) * g->Q * g->pitch);
     a.nodes = static_cast<unsigned>(g->N);
     a.cells = rest ? 0u : static_cast<unsigned>((g->N + CELL - 1) / CELL);
     a.cell_kind = g->d_kind.as<uint8_t>();
@@ -1078,6 +1072,9 @@ wake_grid* wake_grid_create(int q, int nx, int ny, int nz, float tau, int storag
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&g->side, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&g->ev_fork, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&g->ev_join, cudaEventDisableTiming);
+    int dev = 0;
+    if (e == cudaSuccess) e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&g->l2_bytes, cudaDevAttrL2CacheSize, dev);
     const std::size_t sb = g->elem * static_cast<std::size_t>(q) * g->pitch;
     if (e == cudaSuccess) e = g->A.ensure(sb);
     if (e == cudaSuccess) e = g->B.ensure(sb);

@@ -139,6 +139,7 @@ struct wake_grid {
     // reuse a destroyed grid's address for the old one.
     unsigned long long geom_version = 0;
 
+    int l2_bytes = 0;  // L2 cache of the lattice's device
     int tpb = 0, xchunks = 1, rows = 1, tpb_cells = 64;
     // step kernels: 0 automatic, 1 direct (k_step_cells over the whole lattice), 2 to 4 a bulk kernel for the
     // rows whose every node is a pure gather (ROW_FAST) beside k_step_cells for the other rows (`rest`):
@@ -283,7 +284,7 @@ unsigned long long next_geom_version();
 // Step arguments of one lattice: the direct range and its listed cells, or the rows beside a bulk kernel
 // (buffers left for the caller).
 StepArgs grid_step_args(const wake_grid* g, bool rest = false);
-bool fits_l2(long long bytes);
+bool fits_l2(const wake_grid* g, long long bytes);
 // Its buffers: the state in buf(cur), the step's output in the other one.
 void grid_step_buffers(wake_grid* g, int cur, StepArgs& a);
 // The last step left its force outstanding.

@@ -356,7 +356,9 @@ int wake_grid_get_temperature(wake_grid* g, float* T);
 int wake_grid_set_solid_ellipse(wake_grid* g, float cx, float cy, float a, float b, float angle);
 
 /* Device memory: what the grid holds now, and an upper estimate for a new grid
- * of that shape (state buffers, FP32 initialisation scratch, flags, tables;
+ * of that shape (state buffers, FP32 initialisation scratch, flags, the step
+ * lists of a lattice full of obstacles, tables; the automatic kernel, a force
+ * history of 65536 entries;
  * with_fields bit 0 adds the macroscopic-field scratch, bit 1 a coupled temperature). release_scratch first
  * completes any pending setup (flags, initial collide), then frees the FP32
  * population and field scratch (re-allocated on demand by the readers). A

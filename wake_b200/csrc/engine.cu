@@ -1988,9 +1988,17 @@ long long wake_grid_estimate_bytes(int q, int nx, int ny, int nz, int storage, i
     b += q * pitch * 4;                  // FP32 populations for (re)initialisation
     b += 2 * N + 4 * N;                  // cell types, flags, per-node first curved link
     b += 8ll * ny * nz;                  // row lists
+    // Cells: class bytes; a general cell has CELL records, its list entry, units, slots and the partial sums of two
+    // halves, a listed pure one its list entry and units. A run of n general nodes makes ceil(n / CELL) cells and never
+    // more than its segments, a pure one lists a cell more at either end; between two runs of one kind lies another.
+    // 16-bit lattices may hold a second list, of the rows beside the pipelined row kernel.
+    const long long segs = ((nx + CELL - 1) / CELL) * static_cast<long long>(ny) * nz, cells = N / CELL + 1;
+    const long long general = std::min(segs, cells + segs / 2), ends = cells + segs + 1;
+    const int lists = storage == WAKE_STORE_F32 ? 1 : 2;
+    b += segs + cells + lists * (general * (16 * CELL + 16 + 2 * 4 + 2 * 4 + 2 * 2 * 3 * 8) + ends * (16 + 2 * 4));
     if (with_fields) b += 5 * 4 * N;     // rho, ux, uy, uz, speed
     if (thermal) b += 3 * 5 * 4 * pitch;  // coupled temperature: two state buffers and the start-up populations
-    return b + (1ll << 20);              // history ring, slots and small tables
+    return b + (2ll << 20);              // history ring (65536 entries) and small tables
 }
 
 int wake_grid_release_scratch(wake_grid* g) {

@@ -1,4 +1,5 @@
-"""Arithmetic of the step kernels that runs on the host too: the cells' indexes, the division of the Zou-He faces."""
+"""Arithmetic of the step kernels that runs on the host too: the cells' indexes, the division of the Zou-He faces,
+the stress behind the packed BGK kernel's Smagorinsky tau."""
 import shutil
 import subprocess
 from pathlib import Path
@@ -37,4 +38,10 @@ def test_inside_cells_read_their_plane_only(reach, q, nx, ny, nz):
 def test_division_by_a_constant(tmp_path):
     """By 3 and 6 over every 251st float (every 7th of the smallest), the zeros, the largest, infinity and NaN."""
     r = subprocess.run([str(_compile("by_const", tmp_path))], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout
+
+
+def test_stress_of_the_packed_bgk_kernel(tmp_path):
+    """Its error against FP64 is no larger than the one-node kernels' on the same nodes."""
+    r = subprocess.run([str(_compile("bgk_stress", tmp_path))], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stdout

@@ -16,6 +16,7 @@ import oracle  # noqa: E402
 
 STEPS = 20
 TAU = 0.56
+SMAG = 0.6  # the eddy viscosity is then a few per cent of the flow's
 GRIDS = {9: wb.LatticeGrid2D, 19: wb.LatticeGrid3D, 27: wb.LatticeGrid3DQ27}
 
 
@@ -50,7 +51,7 @@ def _step_both(q, size, types, collision, les=False, force=(0.0, 0.0, 0.0), wall
     if mem is not None:
         g.enable_forces(*mem)
     gz = {} if q == 9 else {"gz": force[2]}
-    g.step(collision, gx=force[0], gy=force[1], use_les=les, smag_const=0.17, n=steps, **gz)
+    g.step(collision, gx=force[0], gy=force[1], use_les=les, smag_const=SMAG, n=steps, **gz)
     g.synchronize()
     out = [g]
     for prec in (32, 64):
@@ -58,7 +59,7 @@ def _step_both(q, size, types, collision, les=False, force=(0.0, 0.0, 0.0), wall
         kw = {} if wall is None else {"u_wall": wall}
         if mem is not None:
             kw.update(mem=1, center=mem[:3], r_max=mem[3])
-        o.configure(collision=collision, tau=tau, les=int(les), cs_smag=0.17, g=force, periodic_y=int(periodic[0]),
+        o.configure(collision=collision, tau=tau, les=int(les), cs_smag=SMAG, g=force, periodic_y=int(periodic[0]),
                     periodic_z=int(periodic[1]), **kw)
         o.set_cell_types(types)
         o.set_state(f0)
@@ -94,6 +95,63 @@ def test_pure_run_ends_within_the_last_inner_row(q, size, solid, collision):
     types = np.zeros((nz, ny, nx), np.uint8)
     types[solid[2], solid[1], solid[0]] = wb.SOLID
     _check(q, size, types, collision)
+
+
+def _walls(nx, ny, nz):
+    """A block of solid cells inside and one that crosses the x faces."""
+    types = np.zeros((nz, ny, nx), np.uint8)
+    types[nz // 3:nz // 3 + 3, ny // 2:ny // 2 + 3, nx // 4:nx // 4 + 5] = wb.SOLID
+    types[0, 0, -1] = types[0, 0, 0] = wb.SOLID
+    return types
+
+
+MODELS = [(wb.BGK, False), (wb.BGK, True), (wb.TRT, True), (wb.MRT, False), (wb.MRT, True)]
+
+
+@pytest.mark.parametrize("collision,les", MODELS)
+@pytest.mark.parametrize("q", [19, 27])
+@pytest.mark.parametrize("force", [(0.0, 0.0, 0.0), (2e-5, -1e-5, 3e-5)])
+def test_models_over_walls(q, force, collision, les):
+    """Every collision model with and without Smagorinsky and body force, over general cells of the 3D lattices."""
+    size = (70, 12, 9)
+    _check(q, size, _walls(*size), collision, les=les, force=force, mem=(19.0, 7.0, 4.0, 8.0))
+
+
+@pytest.mark.parametrize("collision,les", MODELS)
+@pytest.mark.parametrize("force", [(0.0, 0.0, 0.0), (2e-5, -1e-5, 0.0)])
+def test_models_over_walls_2d(force, collision, les):
+    size = (99, 33, 1)
+    types = np.zeros((1, 33, 99), np.uint8)
+    types[0, 12:17, 30:34] = wb.SOLID
+    _check(9, size, types, collision, les=les, force=force, mem=(31.0, 14.0, 0.0, 8.0))
+
+
+@pytest.mark.parametrize("collision", [wb.BGK, wb.TRT, wb.MRT])
+@pytest.mark.parametrize("q", [9, 19, 27])
+def test_moving_wall(q, collision):
+    size = (70, 12, 1 if q == 9 else 9)
+    types = _walls(*size) if q != 9 else np.zeros(size[::-1], np.uint8)
+    types[:, -1, :] = wb.MOVING_WALL
+    _check(q, size, types, collision, wall=(0.05, 0.0, 0.0 if q == 9 else 0.02), periodic=(False, q != 9))
+
+
+@pytest.mark.parametrize("collision", [wb.BGK, wb.TRT, wb.MRT])
+def test_moving_curved_links(collision):
+    """Links of a sphere that turns: their moving-wall terms, for delta below and above one half."""
+    size = nx, ny, nz = 66, 14, 12
+    at, radius = (20.0, 7.0, 6.0), 3.3
+    z, y, x = np.meshgrid(np.arange(nz), np.arange(ny), np.arange(nx), indexing="ij")
+    types = ((x - at[0]) ** 2 + (y - at[1]) ** 2 + (z - at[2]) ** 2 <= radius ** 2).astype(np.uint8) * wb.SOLID
+    g = wb.LatticeGrid3D(nx, ny, nz, TAU)
+    g.set_cell_types(types)
+    g.build_curved_sphere_links(*at, radius)
+    node, direction, delta = g.curved_links()
+    g.close()
+    assert (delta < 0.5).any() and (delta >= 0.5).any()
+    rx, ry = node % nx - at[0], (node // nx) % ny - at[1]
+    uw = np.stack([-0.01 * ry, 0.01 * rx, np.full(len(node), 0.005)], axis=1).astype(np.float32)
+    uw[::3] = 0.0  # and links at rest among them
+    _check(19, size, types, collision, links=(node, direction, delta, uw), periodic=(True, True), mem=(*at, 6.0))
 
 
 def test_moments_into_a_buffer_that_is_too_short_are_refused():

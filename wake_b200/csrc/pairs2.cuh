@@ -16,7 +16,7 @@
 //     rho = 1 + w_0 h_0 + sum w S,   j = sum c w D,
 //     S_eq = 2 rho (1 - 1.5 u^2 + 4.5 (c.u)^2) - 2,   D_eq = 6 rho (c.u),
 // and the same update in h, so stored values are used without decoding.
-// gy is the y body force of the two nodes (a coupled temperature gives each its own; otherwise P.g[1] twice)
+// gy (FP32 forms) is the y body force of the two nodes, P.g[1] twice,
 // and `forced` whether any body force acts.
 // Every rounding is explicit (packed ops are never contracted by the compiler).
 #pragma once
@@ -48,10 +48,10 @@ __device__ __forceinline__ float2 acc_cw(float2 acc, int c, float w, float2 v) {
 }
 __host__ __device__ __forceinline__ float2 neg2(float2 a) { return make_float2(-a.x, -a.y); }
 
-// Shifted populations.
+// Shifted populations. The body force is P.g for both nodes (as packed gy it cost the pipelined row kernel 4 more spilled
+// values a thread: D3Q19 F16 256^3 box with Smagorinsky 267 us a step, 257 so).
 template <int Q, bool LES>
-__device__ __forceinline__ void trt_pairs2_h(float2* f, const Physics& P, const float2 gy, const bool forced, float2& rho,
-                                             float2 u[3]) {
+__device__ __forceinline__ void trt_pairs2_h(float2* f, const Physics& P, const bool forced, float2& rho, float2 u[3]) {
     using L = Lat<Q>;
     constexpr int NP = (Q - 1) / 2;
     float2 s[NP], d[NP];
@@ -76,7 +76,7 @@ __device__ __forceinline__ void trt_pairs2_h(float2* f, const Physics& P, const 
     const float* g = P.g;
     const float2 hr = mul2(bc2(0.5f), r);
     u[0] = mul2(forced ? fma2(hr, bc2(g[0]), jx) : jx, inv);
-    u[1] = mul2(forced ? fma2(hr, gy, jy) : jy, inv);
+    u[1] = mul2(forced ? fma2(hr, bc2(g[1]), jy) : jy, inv);
     u[2] = mul2(forced ? fma2(hr, bc2(g[2]), jz) : jz, inv);
     const float2 u2 = fma2(u[2], u[2], fma2(u[1], u[1], mul2(u[0], u[0])));
     const float2 a0 = fma2(bc2(-1.5f), u2, bc2(1.0f));
@@ -129,7 +129,7 @@ __device__ __forceinline__ void trt_pairs2_h(float2* f, const Physics& P, const 
     float2 ug;
     float2 ps, pa;
     if (forced) {
-        ug = fma2(u[2], bc2(g[2]), fma2(u[1], gy, mul2(u[0], bc2(g[0]))));
+        ug = fma2(u[2], bc2(g[2]), fma2(u[1], bc2(g[1]), mul2(u[0], bc2(g[0]))));
         ps = fma2(bc2(-1.0f), hs, bc2(1.0f));  // 1 - omega_s / 2
         pa = fma2(bc2(-1.0f), ha, bc2(1.0f));
         // Guo term of the rest population: (1 - omega_s/2) w_0 rho (-3 u.g)
@@ -154,13 +154,13 @@ __device__ __forceinline__ void trt_pairs2_h(float2* f, const Physics& P, const 
         {
             // Guo forcing of the pair (collide_trt_t in lattice.cuh): even part
             // (1 - omega_s/2) w rho (-3 u.g + 9 (c.u)(c.g)), odd part (1 - omega_a/2) w rho 3 (c.g)
-            float2 cg = bc2(L::cx(q) > 0 ? g[0] : (L::cx(q) < 0 ? -g[0] : 0.0f));
-            cg = acc_c(cg, L::cy(q), gy);
-            cg = acc_c(cg, L::cz(q), bc2(g[2]));
+            float cg = L::cx(q) > 0 ? g[0] : (L::cx(q) < 0 ? -g[0] : 0.0f);
+            if (L::cy(q)) cg = __fadd_rn(cg, L::cy(q) > 0 ? g[1] : -g[1]);
+            if (L::cz(q)) cg = __fadd_rn(cg, L::cz(q) > 0 ? g[2] : -g[2]);
             float2 cu = fma2(bc2(float(L::cz(q))), u[2], fma2(bc2(float(L::cy(q))), u[1], mul2(bc2(float(L::cx(q))), u[0])));
             const float2 fr = r;
-            const float2 ev = mul2(mul2(ps, fr), fma2(mul2(bc2(9.0f), cg), cu, mul2(bc2(-3.0f), ug)));
-            const float2 od = mul2(mul2(pa, fr), mul2(bc2(3.0f), cg));
+            const float2 ev = mul2(mul2(ps, fr), fma2(bc2(__fmul_rn(9.0f, cg)), cu, mul2(bc2(-3.0f), ug)));
+            const float2 od = mul2(mul2(pa, fr), bc2(__fmul_rn(3.0f, cg)));
             A = sub2(A, ev);
             B = sub2(B, od);
         }
@@ -284,7 +284,7 @@ __device__ __forceinline__ void trt_pairs2_f(float2* f, const Physics& P, const 
 template <int Q, bool LES, bool HS>
 __device__ __forceinline__ void trt_pairs2(float2* f, const Physics& P, const float2 gy, const bool forced, float2& rho,
                                            float2 u[3]) {
-    if constexpr (HS) trt_pairs2_h<Q, LES>(f, P, gy, forced, rho, u);
+    if constexpr (HS) trt_pairs2_h<Q, LES>(f, P, forced, rho, u);
     else trt_pairs2_f<Q, LES>(f, P, gy, forced, rho, u);
 }
 

@@ -527,8 +527,9 @@ __device__ __forceinline__ void listed_unit(const StepArgs& a, const At& at, uns
 }
 
 // Register budgets (blocks of up to 64 threads): common.cuh.
-template <int Q, int COLL, int S, bool TH, bool BATCH>
+template <int Q, int COLL, int S, bool LES, bool TH, bool BATCH>
 constexpr int cell_min_blocks() {
+    if (Q == 27 && COLL == COLL_MRT && S == STORE_F32 && (LES || BATCH)) return WK_PAIRS27_MIN_BLOCKS;
     if (!pure_pairs<Q, COLL, S>() || (TH && !BATCH)) return Q == 9 ? (TH ? 16 : 18) : (Q == 19 ? 12 : 8);
     if (Q != 9) return WK_PAIRS_MIN_BLOCKS;
     return BATCH ? WK_PAIRS9_BATCH_MIN_BLOCKS : WK_PAIRS9_MIN_BLOCKS;
@@ -576,7 +577,7 @@ __device__ __forceinline__ void after_last_step() {
 
 // One step of one lattice: the listed cells and the pure cells of cells 0 .. cells - 1.
 template <int Q, int COLL, int S, bool LES, bool TH>
-__global__ void __launch_bounds__(WK_FAST_MAX_THREADS, (cell_min_blocks<Q, COLL, S, TH, false>())) k_step_cells(const StepArgs a) {
+__global__ void __launch_bounds__(WK_FAST_MAX_THREADS, (cell_min_blocks<Q, COLL, S, LES, TH, false>())) k_step_cells(const StepArgs a) {
     after_last_step();
     const OneLattice<Q, typename Codec<S>::T> at{a, read_policy(a.evict_first)};
     constexpr unsigned W = pure_units<Q, COLL, S, TH>();
@@ -633,7 +634,7 @@ __device__ __forceinline__ OneMember<Q, typename Codec<S>::T> batch_at(const Bat
 }
 
 template <int Q, int COLL, int S, bool LES, bool TH>
-__global__ void __launch_bounds__(WK_FAST_MAX_THREADS, (cell_min_blocks<Q, COLL, S, TH, true>()))
+__global__ void __launch_bounds__(WK_FAST_MAX_THREADS, (cell_min_blocks<Q, COLL, S, LES, TH, true>()))
     k_step_cells_batch(const BatchArgs b) {
     after_last_step();
     constexpr unsigned W = pure_units<Q, COLL, S, false>();

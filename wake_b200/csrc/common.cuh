@@ -12,6 +12,11 @@
 // 96 registers (20 warps) 119.1, 120.1, 9.0. D2Q9 carries half the values: 64 registers and 32 warps (2048x1024:
 // 22.0 us, 25.1 with 96 registers); 80 where a batch's arguments have to be read (60 channels: 52.0 us a step, 56.7
 // with 96 registers, 53.5 with 72).
+// The FP32 D3Q27 MRT takes 168 with Smagorinsky's tau and in a batch: with 128 it spills 2.2 KB a thread (256^3 box with
+// Smagorinsky 664 us a step, 920 with 128; batch of two 160^3 boxes 345, 473).
+#ifndef WK_PAIRS27_MIN_BLOCKS
+#define WK_PAIRS27_MIN_BLOCKS 5
+#endif
 #ifndef WK_FAST_MAX_THREADS
 #define WK_FAST_MAX_THREADS 64
 #endif

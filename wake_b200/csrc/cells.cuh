@@ -116,6 +116,7 @@ __device__ __forceinline__ void cell_t5(const Thermal& th, const float* tin, lon
 // (constant memory, so an address is one multiply-add on the node index), for any lattice size.
 template <int Q, class T>
 struct OneLattice {
+    static constexpr bool UNIFORM = Q != 9;  // one node per thread: addresses from the warp's first node (cell_one)
     const StepArgs& a;
     L2Policy ld;
     __device__ __forceinline__ const T* in(int q, unsigned e) const { return static_cast<const T*>(a.in[q]) + e; }
@@ -129,6 +130,7 @@ struct OneLattice {
 // two buffers (the host steps members with Q * pitch >= 2^32 by themselves).
 template <int Q, class T>
 struct OneMember {
+    static constexpr bool UNIFORM = false;
     const T* f;
     T* g;
     const float* t_in;
@@ -399,9 +401,10 @@ __device__ __forceinline__ void cell_pairs(const StepArgs& a, const At& at, uint
     }
 }
 
-// Half a cell (32 nodes), one node per thread.
+// Half a cell (32 nodes), one node per thread; known: how a pure one gathers (cell_gather), below 0 if to be found.
 template <int Q, int COLL, int S, bool LES, bool TH, bool PURE, class At>
-__device__ __forceinline__ void cell_one(const StepArgs& a, const At& at, uint4 cell, int entry, bool zh, int half) {
+__device__ __forceinline__ void cell_one(const StepArgs& a, const At& at, uint4 cell, int entry, bool zh, int half,
+                                         int known = -1) {
     using L = Lat<Q>;
     using C = Codec<S>;
     using T = typename C::T;
@@ -409,6 +412,10 @@ __device__ __forceinline__ void cell_one(const StepArgs& a, const At& at, uint4 
     const int count = static_cast<int>(cell.y & 0xffu);
     const int lane = threadIdx.x & 31, o = 32 * half + lane;
     unsigned i = i0 + o;
+    // UNIFORM: a plane's address is a uniform one, of the half cell's first node, and the lane's 32-bit offset, which
+    // takes no instruction per plane (D3Q27 F16 MRT 256^3 box: 621 -> 595 us a step). Elsewhere it was up to 5 % slower
+    // (D2Q9) or 12 % (a batch of two 160^3 F16 boxes, whose bases are not parameters: 216 -> 241).
+    const unsigned at0 = At::UNIFORM ? i0 + 32 * half : i, off = At::UNIFORM ? lane : 0;
     bool v = o < count;
     uint4 r = make_uint4(0u, 0u, 0u, 0u);
     bool mem = false;  // uniform: the half cell holds momentum-exchange nodes
@@ -425,15 +432,24 @@ __device__ __forceinline__ void cell_one(const StepArgs& a, const At& at, uint4 
     const long long P = a.geo.pitch;
     PullOffsets d;
     float f[Q];
-    const CellGather way = PURE ? cell_gather<Q>(a.geo, i0, count) : FACES;  // uniform
+    const int way = !PURE ? FACES : (known >= 0 ? known : cell_gather<Q>(a.geo, i0, count));  // uniform
     if (PURE && way == INSIDE) {
 #pragma unroll
-        for (int q = 0; q < Q; ++q) f[q] = load_f<S>(at.pull(q, i), L::w(q), at.ld);
+        for (int q = 0; q < Q; ++q) f[q] = load_f<S>(at.pull(q, at0) + off, L::w(q), at.ld);
     } else if (PURE && way == ROW_ENDS) {
         const unsigned nx = a.geo.nx, x = i - a.geo.by_nx.quot(i) * nx;
-        const unsigned im = x == 0u ? i + nx : i, ip = x == nx - 1u ? i - nx : i;  // c_x = +1 / -1
+        if constexpr (At::UNIFORM) {
+            const unsigned om = x == 0u ? off + nx : off, op = x == nx - 1u ? off : off + nx;  // c_x = +1, and -1 from at0 - nx
 #pragma unroll
-        for (int q = 0; q < Q; ++q) f[q] = load_f<S>(at.pull(q, L::cx(q) > 0 ? im : (L::cx(q) < 0 ? ip : i)), L::w(q), at.ld);
+            for (int q = 0; q < Q; ++q)
+                f[q] = load_f<S>(at.pull(q, L::cx(q) < 0 ? at0 - nx : at0) + (L::cx(q) > 0 ? om : (L::cx(q) < 0 ? op : off)),
+                                 L::w(q), at.ld);
+        } else {
+            const unsigned im = x == 0u ? i + nx : i, ip = x == nx - 1u ? i - nx : i;  // c_x = +1 / -1
+#pragma unroll
+            for (int q = 0; q < Q; ++q)
+                f[q] = load_f<S>(at.pull(q, L::cx(q) > 0 ? im : (L::cx(q) < 0 ? ip : i)), L::w(q), at.ld);
+        }
     } else if (PURE) {
         d = pull_offsets<Q>(a.geo, i);
 #pragma unroll
@@ -490,7 +506,7 @@ __device__ __forceinline__ void cell_one(const StepArgs& a, const At& at, uint4 
     if (!(rho > 0.0f) || !(fabsf(u[0]) < 1e30f)) atomicOr(a.status, ERR_NONFINITE);
     collide<Q, COLL, LES>(f, rho, u, ph);
 #pragma unroll
-    for (int q = 0; q < Q; ++q) store_f<S>(at.out(q, i), f[q], L::w(q));
+    for (int q = 0; q < Q; ++q) store_f<S>(at.out(q, at0) + off, f[q], L::w(q));
     if constexpr (TH) {
         if (a.th.on) {
             collide_t5(t5, Tn, u, a.th.omega_t);
@@ -535,12 +551,12 @@ constexpr int cell_min_blocks() {
     return BATCH ? WK_PAIRS9_BATCH_MIN_BLOCKS : WK_PAIRS9_MIN_BLOCKS;
 }
 
-// The work units of a warp of the pure blocks (block index b of them): `run` units (cells, or half cells), those
+// The work units of warp `warp` of the pure blocks (block index b of them): `run` units (cells, or half cells), those
 // of a block's warps adjacent. load(u), the unit's class or entry, goes out while the unit before it is stepped.
 template <class Load, class Step>
-__device__ __forceinline__ void walk(unsigned b, unsigned units, unsigned run, Load load, Step step) {
+__device__ __forceinline__ void walk(unsigned b, unsigned warp, unsigned units, unsigned run, Load load, Step step) {
     const unsigned wpb = blockDim.x >> 5;
-    unsigned u = b * (wpb * run) + (threadIdx.x >> 5);
+    unsigned u = b * (wpb * run) + warp;
     if (u >= units) return;
     auto d = load(u);
 #pragma unroll 1
@@ -591,14 +607,29 @@ __global__ void __launch_bounds__(WK_FAST_MAX_THREADS, (cell_min_blocks<Q, COLL,
             listed_unit<Q, COLL, S, LES, TH>(a, at, __ldg(a.units + k));
         return;
     }
+    // 3D, one node per thread: a warp with several half cells takes both halves of a cell in turn and classifies it once
+    // (256^3 boxes, F16 MRT: D3Q19 454 -> 420 us a step, D3Q27 667 -> 621; D2Q9 2048x1024 MRT 26.9 -> 27.9, so not there)
+    constexpr bool TURN = W == 2u && Q != 9;
+    const unsigned per = TURN ? min(a.run, W) : 1u;
+    unsigned warp = threadIdx.x >> 5;
+    if constexpr (TURN) warp = __shfl_sync(0xffffffffu, warp, 0);  // known to the compiler as the warp's
     walk(
-        block, a.cells * W, a.run, [&](unsigned u) { return static_cast<unsigned>(__ldg(a.cell_kind + u / W)); },
+        block, warp, a.cells * W / per, a.run / per, [&](unsigned u) { return static_cast<unsigned>(__ldg(a.cell_kind + u * per / W)); },
         [&](unsigned u, unsigned kind) {
             if (!(kind & CELL_PURE)) return;
-            const unsigned i0 = u / W * CELL;
+            const unsigned i0 = u * per / W * CELL;
             const uint4 cell = make_uint4(i0, min(CELL + 0u, a.nodes - i0), 0u, 0u);
-            if constexpr (W == 1u) cell_pairs<Q, COLL, S, LES, true>(a, at, cell, -1, (kind & CELL_ZH) != 0);
-            else cell_one<Q, COLL, S, LES, TH, true>(a, at, cell, -1, (kind & CELL_ZH) != 0, u % W);
+            if constexpr (W == 1u) {
+                cell_pairs<Q, COLL, S, LES, true>(a, at, cell, -1, (kind & CELL_ZH) != 0);
+            } else if constexpr (!TURN) {
+                cell_one<Q, COLL, S, LES, TH, true>(a, at, cell, -1, (kind & CELL_ZH) != 0, u % W);
+            } else {
+                const int way = cell_gather<Q>(a.geo, i0, cell.y);
+                const unsigned h0 = u * per % W;
+#pragma unroll 1
+                for (unsigned h = h0; h < h0 + per; ++h)
+                    cell_one<Q, COLL, S, LES, TH, true>(a, at, cell, -1, (kind & CELL_ZH) != 0, static_cast<int>(h), way);
+            }
         });
 }
 
@@ -657,7 +688,7 @@ __global__ void __launch_bounds__(WK_FAST_MAX_THREADS, (cell_min_blocks<Q, COLL,
         return;
     }
     walk(
-        block, b.npure * W, b.run, [&](unsigned u) { return __ldg(b.pure + u / W); },
+        block, threadIdx.x >> 5, b.npure * W, b.run, [&](unsigned u) { return __ldg(b.pure + u / W); },
         [&](unsigned u, uint2 r) {
             const BatchDom& d = b.dom[r.x & 0xffffffu];
             const StepArgs& a = d.a;

@@ -180,10 +180,12 @@ unsigned blocks_of(unsigned units, int tpb) {
 // still fill the device (148 SMs, 10 or more blocks each) several times over: a block's start costs about a tenth
 // of a one-unit block's life (D3Q19 FP32 160^3: 110.5 us with one, 106.6 with two, 113 with eight); smaller
 // lattices need the blocks to even out the end (97^3: 27.3 / 26.8 / 29.8; D2Q9 1024x512, 8192 blocks of one unit: BGK
-// 9.4 / 8.5, MRT 9.0 / 7.5).
-unsigned plan(unsigned units, int tpb, unsigned list_blocks, unsigned& run, unsigned& spread) {
+// 9.4 / 8.5, MRT 9.0 / 7.5). `four`: four units from 74,000 blocks, on D3Q19 and FP16C lattices (256^3 box, two / four:
+// D3Q19 FP32 TRT 414 / 399, F16 MRT 417 / 412, D3Q27 FP16C MRT 733 / 721; D3Q27 F16 BGK 588 / 599 and FP32 BGK
+// 568 / 570, so not there).
+unsigned plan(unsigned units, int tpb, unsigned list_blocks, bool four, unsigned& run, unsigned& spread) {
     unsigned blocks = blocks_of(units, tpb);
-    run = blocks >= 148u * 40u ? 2u : 1u;
+    run = blocks >= 148u * 500u && four ? 4u : (blocks >= 148u * 40u ? 2u : 1u);
     blocks = list_blocks + (blocks + run - 1u) / run;
     spread = 0;
     while (list_blocks && (static_cast<unsigned long long>(list_blocks) << (spread + 1)) <= blocks / 5ull * 3ull) ++spread;
@@ -208,13 +210,13 @@ void launch_step(void (*kernel)(A), unsigned blocks, int tpb, cudaStream_t st, c
 template <int C, int S, bool LES, bool TH>
 void cells_one(StepArgs& a, int tpb, cudaStream_t st) {
     a.list_blocks = blocks_of(a.nunits + (a.mem.enabled ? 1u : 0u), tpb);
-    const unsigned blocks = plan(a.cells * pure_units<kQ, C, S, TH>(), tpb, a.list_blocks, a.run, a.spread);
+    const unsigned blocks = plan(a.cells * pure_units<kQ, C, S, TH>(), tpb, a.list_blocks, kQ == 19 || S == STORE_F16C, a.run, a.spread);
     if (blocks) launch_step(k_step_cells<kQ, C, S, LES, TH>, blocks, tpb, st, a, a.early != 0);
 }
 template <int C, int S, bool LES, bool TH>
 void batch_one(BatchArgs& b, int tpb, cudaStream_t st) {
     b.list_blocks = blocks_of(b.nlisted, tpb);
-    const unsigned blocks = plan(b.npure * pure_units<kQ, C, S, false>(), tpb, b.list_blocks, b.run, b.spread);
+    const unsigned blocks = plan(b.npure * pure_units<kQ, C, S, false>(), tpb, b.list_blocks, false, b.run, b.spread);
     if (blocks) launch_step(k_step_cells_batch<kQ, C, S, LES, TH>, blocks, tpb, st, b, true);
 }
 template <int C, int S, bool LES>

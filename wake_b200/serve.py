@@ -151,12 +151,12 @@ def job_bytes(job: Job, storage: str) -> int:
     return int(lib.wake_grid_estimate_bytes(q, nx, ny, nz, STORAGE[storage], flags))
 
 
-# Sphere jobs at least this wide step alone through the single-lattice kernels (with CUDA graphs
-# of SOLO_GRAPH_STEPS steps): measured on one B200 (FP32, TRT + LES), n = 112..160 run at 24-29k
-# MLUPS alone, within 10% of a batch of equal jobs or faster, while smaller jobs gain 1.3-2.3x from
-# batching (device rates measured by bench.py serving_rates). Solo jobs keep the batch's row lists
-# short, and those lists are rebuilt whenever the batch's membership changes.
-SOLO_MIN_EDGE = 112
+# Sphere jobs at least this wide step alone through the single-lattice kernel (with CUDA graphs of SOLO_GRAPH_STEPS
+# steps). Measured on one B200 (FP32, TRT + LES; MLUPS alone / in a batch of equal jobs of about 4.2 M nodes, bench.py
+# serving_rates): edge 48 18.6k / 28.3k, 64 32.4k / 32.0k, 80 36.4k / 31.8k, 96 35.3k / 33.1k, 160 36.8k / 34.7k. The mix
+# of mixed_jobs(150, 64 jobs/s): 15.33 sims/s with the line at 64 or 80, 15.13 at 112, 14.50 with every job batched.
+# Solo jobs also keep the batch's cell lists short, and those lists are rebuilt whenever the batch's membership changes.
+SOLO_MIN_EDGE = 64
 SOLO_GRAPH_STEPS = 20
 
 
@@ -167,8 +167,8 @@ def _class_key(job: Job):
 
 
 class _Solo:
-    """A job large enough to fill the device by itself, stepped through its own grid on its own
-    stream (the batch interface the serving loop uses)."""
+    """A job that steps faster by itself, through its own grid on its own stream (the batch interface
+    the serving loop uses)."""
 
     def __init__(self):
         self.g = None
@@ -278,7 +278,7 @@ class Server:
                 pending.popleft()
                 g, case = _start(job, self.storage)
                 g._apply_model(case.collision, case.les, case.cs_smag)
-                # flags, row lists and the initial collide on the job's own stream, then free the
+                # flags, cell lists and the initial collide on the job's own stream, then free the
                 # FP32 start-up scratch: all of it overlaps the batches' running tick
                 check(lib.wake_grid_release_scratch(g.handle))
                 staged.append((job, g, case, need, now()))

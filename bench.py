@@ -343,9 +343,8 @@ STEPS_PER_SIM = 5000
 def batched_leg(storage, n_domains=512, steps=STEPS_PER_SIM, warmup=20, baseline_jobs=16):
     """Sims/s of the ellipse sweep advanced as one batch, and of the same jobs launched per job.
 
-    Batched: every domain resident, one bulk + one general launch + one force
-    reduction per step for all 512 domains, CUDA graphs of 20 steps, bulk block
-    size from the autotuner. Per job: the first `baseline_jobs` domains run one
+    Batched: every domain resident, one launch per step for all 512 domains, CUDA
+    graphs of 20 steps, block size from the autotuner. Per job: the first `baseline_jobs` domains run one
     after another through their own grid with plain launches (the single-lattice
     API used once per job). Both time `steps` steps with CUDA events after warm-up;
     setup is outside both timed regions."""

@@ -371,9 +371,8 @@ long long wake_grid_estimate_bytes(int q, int nx, int ny, int nz, int storage, i
 int wake_grid_release_scratch(wake_grid* g);
 
 /* ------------------------------------------------------------------ batches
- * A batch advances many resident grids together: one bulk launch over the
- * pure-gather rows of every member, one launch over the remaining rows and one
- * momentum-exchange reduction per step, whatever the members' sizes. Members
+ * A batch advances many resident grids together: one launch per step over the
+ * cells of every member, whatever the members' sizes. Members
  * share the lattice and storage (checked by add) and the collision model and LES
  * switch (checked by step); sizes, tau, boundaries, geometry and force monitors
  * are per member. A member stays an ordinary grid: its readers (populations,
@@ -396,6 +395,8 @@ int wake_batch_get_block(wake_batch* b);
 int wake_batch_set_kernel(wake_batch* b, int variant);
 int wake_batch_step(wake_batch* b, int n);
 int wake_batch_synchronize(wake_batch* b);        /* first member error, if any */
+/* bulk_rows: cells of pure gathers, up to 64 nodes each; general_rows: warps' units of the other cells, and one per
+ * member with forces; members of 2^32 or more values, which step by their own launches, count in the launches only. */
 int wake_batch_info(wake_batch* b, long long* nodes, int* bulk_rows, int* general_rows, int* launches_per_step);
 /* Times `steps` real steps per bulk block size (those of 32, 64, 128, 256 within
  * the build's bound, 64 by default) and keeps the fastest; members advance

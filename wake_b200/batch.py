@@ -2,8 +2,7 @@
 
 A ``Batch`` holds grids of one lattice and storage (``LatticeGrid2D`` /
 ``LatticeGrid3D`` / ``LatticeGrid3DQ27`` objects) and advances all of them with
-one bulk launch, one general launch and one force reduction per step,
-whatever their sizes. Each member keeps its own geometry, tau, boundaries and
+one launch per step, whatever their sizes. Each member keeps its own geometry, tau, boundaries and
 force history and is read through its usual accessors between steps; its
 results are the ones it gets when stepped alone.
 
@@ -89,7 +88,7 @@ class Batch:
         return check(lib.wake_batch_get_block(self._h))
 
     def autotune(self, steps: int = 20) -> int:
-        """Pick the bulk block size by timing real steps (members advance `steps` per size tried)."""
+        """Pick the block size by timing real steps (members advance `steps` per size tried)."""
         best = ctypes.c_int()
         check(lib.wake_batch_autotune(self._h, steps, ctypes.byref(best)))
         return best.value
@@ -104,6 +103,8 @@ class Batch:
         check(lib.wake_batch_synchronize(self._h))
 
     def info(self) -> dict:
+        """Members, nodes and kernel launches per step; ``bulk_rows`` counts the cells of pure gathers and
+        ``general_rows`` the warps' units of the others (wake_batch_info)."""
         nodes, fr, gr, lps = ctypes.c_longlong(), ctypes.c_int(), ctypes.c_int(), ctypes.c_int()
         check(lib.wake_batch_info(self._h, ctypes.byref(nodes), ctypes.byref(fr), ctypes.byref(gr), ctypes.byref(lps)))
         return {"members": len(self._members), "nodes": nodes.value, "bulk_rows": fr.value, "general_rows": gr.value,

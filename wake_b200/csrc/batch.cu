@@ -36,7 +36,7 @@ struct wake_batch {
     int coll = 0, les = 0;
     int parity = 0;  // batch steps taken, mod 2
 
-    // row lists are rebuilt when the members or any member's geometry change
+    // cell lists are rebuilt when the members or any member's geometry change
     std::vector<std::pair<const wake_grid*, unsigned long long>> layout;
     unsigned shape = 0;  // bumped when launch shapes or table addresses change
     // host seconds spent in wake_batch_step: preparing members and tables, capturing and
@@ -308,7 +308,7 @@ int wake_batch_set_block(wake_batch* b, int threads_bulk, int threads_general) {
     if (!valid_batch(b)) return WAKE_ERR_INVALID;
     if (threads_bulk < 32 || threads_bulk > WK_FAST_MAX_THREADS || threads_bulk % 32 || threads_general < 32 ||
         threads_general > 512 || threads_general % 32)
-        return set_error(WAKE_ERR_INVALID, "wake_batch_set_block: bulk 32..256 (at most the fast kernels' bound), "
+        return set_error(WAKE_ERR_INVALID, "wake_batch_set_block: bulk 32 or 64 (the step kernel's bound), "
                                            "general 32..512, multiples of 32");
     b->tpb = threads_bulk;  // one launch steps the general rows too
     b->drop_graph();
@@ -410,8 +410,8 @@ int wake_batch_info(wake_batch* b, long long* nodes, int* bulk_rows, int* genera
     return WAKE_OK;
 }
 
-// Time `steps` real steps for each bulk block size of {32, 64, 128, 256} within the
-// kernels' launch bound (plain launches, CUDA events on the batch stream) and keep
+// Time `steps` real steps for each block size of {32, 64, 128, 256} within the
+// kernel's launch bound (plain launches, CUDA events on the batch stream) and keep
 // the fastest. The members advance `steps` per size tried; results do not depend on
 // the block size.
 int wake_batch_autotune(wake_batch* b, int steps, int* best_threads) {

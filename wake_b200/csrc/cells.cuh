@@ -2,8 +2,8 @@
 // warp (two nodes per thread in packed FP32, pairs2.cuh) or two (one node per thread). One launch steps the lattice.
 //
 // Cells ignore the row ends, so nearly every warp is full whatever nx is. Rows cut into 64-node pieces leave lanes
-// idle wherever nx is no multiple of 64 (81-node rows: 64 + 17; 81^3 sphere channel, D3Q19 FP32: 26.2 -> 14.2 us a
-// step, 97^3 38.9 -> 25.1, 160^3 152 -> 111). A node's pull sources are its own index plus one of three x, y
+// idle wherever nx is no multiple of 64 (81-node rows: 64 + 17; 81^3 sphere channel, D3Q19 FP32: 26.2 -> 14.4 us a
+// step, 97^3 38.9 -> 26.1, 160^3 152 -> 112). A node's pull sources are its own index plus one of three x, y
 // and z offsets (the periodic wraps included), so a load costs one or two integer adds.
 //
 // Two kinds of cells. A pure one, all in segments of pure gathers (FL_FAST), reads nothing but its class and the
@@ -149,12 +149,6 @@ struct OneMember {
     __device__ __forceinline__ int cur() const { return c; }
 };
 
-// Decoded value of population q from its stored one (h = f / w - 1 for the 16-bit storages).
-template <int Q, int S>
-__device__ __forceinline__ float to_f(float v, int q) {
-    return S == STORE_F32 ? v : fmaf(Lat<Q>::w(q), v, Lat<Q>::w(q));
-}
-
 // The curved links of a cell (Bouzidi linear interpolation from post-collision values,
 // d3q19_curved.ispc:36-68). They are consecutive in the link array, so the warp evaluates them one per lane,
 // 128 with their loads in flight together, and each node picks its values up from shared memory (`sm`, 128 values
@@ -267,7 +261,7 @@ __device__ __forceinline__ float* link_values() {
 // which leaves with one 32-bit store per plane where the cell starts on an even node. PURE: a pure cell, zh telling
 // whether it holds Zou-He nodes; otherwise the general cell `entry`. The two are compiled apart: the general
 // path's live values would cost the pure one registers, hence loads in flight.
-// Bound by memory: 152 B a node, of which D3Q19 FP32 256x128x128 moves 5.8 TB/s (109.9 us a step;
+// Bound by memory: 152 B a node, of which D3Q19 FP32 256x128x128 moves 5.8 TB/s (110.0 us a step;
 // 118.2 with one warp per row segment).
 template <int Q, int COLL, int S, bool LES, bool PURE, class At>
 __device__ __forceinline__ void cell_pairs(const StepArgs& a, const At& at, uint4 cell, int entry, bool zh) {
@@ -579,8 +573,8 @@ __device__ __forceinline__ void walk(unsigned b, unsigned warp, unsigned units, 
 // one until all are placed (list_blocks << spread is about 60 % of the blocks): the listed cells' latency chain
 // then never holds more than a few of the device's block slots at once, and none of it is left at the end.
 // All of them at the front held half the slots for 20 us on a 160^3 sphere channel. Every other step takes the
-// pure cells from the end (`reverse`): what the last step wrote last is still in L2 (256x128x128: 109.9 -> 108.4 us,
-// 2048x1024 D2Q9: 28.4 -> 26.4 us).
+// pure cells from the end (`reverse`): what the last step wrote last is still in L2 (256x128x128: 112.1 -> 110.0 us, 160^3
+// 113.5 -> 111.8; lattices that are read evict-first are within 2 % either way).
 __device__ __forceinline__ unsigned which_block(unsigned list_blocks, unsigned spread, bool reverse, bool& first) {
     const unsigned b = blockIdx.x, k = b >> spread;
     first = k < list_blocks && (b & ((1u << spread) - 1u)) == 0u;
@@ -590,9 +584,9 @@ __device__ __forceinline__ unsigned which_block(unsigned list_blocks, unsigned s
 
 // A step's launch may start before the step before it has ended (launch_step), as that one's blocks end: wait for its
 // results. The blocks come up and take over where they had the latency of a launch between steps: D2Q9
-// 400x160 in a graph 2.95 -> 2.5 us a step, as plain launches 4.1 -> 2.5 (the host's rate of launches), with a
-// temperature 384x192 5.6 -> 4.0; D3Q19 48^3 sphere 5.9 -> 5.5, 256x128x128 109.9 -> 109.6. Letting the next launch
-// start as soon as every block of this one runs was slower (1024x512 BGK 9.4 / 8.6, temperature 3.2 / 3.0 in graphs).
+// 400x160 in a graph 3.5 -> 3.2 us a step, as plain launches 6.1 -> 3.4 (the host's rate of launches), 1024x512 MRT 7.9 -> 7.6
+// and 10.2 -> 7.8; D3Q19 48^3 sphere 5.95 -> 5.6, 256x128x128 110.4 -> 110.0. Letting the next launch start as
+// soon as every block of this one runs was slower (1024x512 BGK 9.4, 8.6 without, in graphs).
 __device__ __forceinline__ void after_last_step() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }

@@ -1265,7 +1265,7 @@ int wake_grid_enable_thermal(wake_grid* g, float tau_t, float t_ref, float beta_
     g->th.beta_g = beta_g;
     g->th.t_south = t_south;
     g->th.t_north = t_north;
-    g->geom_dirty = true;  // every segment moves to the general path
+    g->geom_dirty = true;  // the units of the cells differ
     g->pending = true;
     g->invalidate_graph();
     if (!g->mt_valid) {  // start from the reference temperature everywhere
@@ -1987,7 +1987,7 @@ long long wake_grid_estimate_bytes(int q, int nx, int ny, int nz, int storage, i
     long long b = 2 * q * pitch * elem;  // state buffers
     b += q * pitch * 4;                  // FP32 populations for (re)initialisation
     b += 2 * N + 4 * N;                  // cell types, flags, per-node first curved link
-    b += 8ll * ny * nz;                  // row lists
+    b += 8ll * ny * nz;                  // row tables
     // Cells: class bytes; a general cell has CELL records, its list entry, units, slots and the partial sums of two
     // halves, a listed pure one its list entry and units. A run of n general nodes makes ceil(n / CELL) cells and never
     // more than its segments, a pure one lists a cell more at either end; between two runs of one kind lies another.

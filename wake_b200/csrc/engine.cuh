@@ -134,7 +134,7 @@ struct wake_grid {
     wk::CellList cells;
     unsigned long long units_version = 0;  // a fresh number whenever units are made (next_geom_version)
     long long cell_nodes = 0;  // nodes of the segments that are not all solid
-    // Identity of the current flags / row lists: a fresh process-wide number at every
+    // Identity of the current flags / cell lists: a fresh process-wide number at every
     // rebuild (next_geom_version), so a batch never takes a new grid that happens to
     // reuse a destroyed grid's address for the old one.
     unsigned long long geom_version = 0;
@@ -244,7 +244,7 @@ struct wake_grid {
         l.count = dev_links;
         return l;
     }
-    Launch launch() const { return Launch{tpb, xchunks, rows, stream, ny, nz, tpb_cells}; }
+    Launch launch() const { return Launch{tpb, xchunks, rows, stream, ny, nz}; }
     int blocks() const { return rows * xchunks; }
 
     void invalidate_graph() { graph_ok = false; }

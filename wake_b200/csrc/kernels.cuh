@@ -18,7 +18,6 @@ struct Launch {
     int rows;      // ny * nz
     cudaStream_t stream;
     int ny, nz;
-    int tpb_cells;  // threads per block of k_step_cells
 };
 
 struct FlagCfg {

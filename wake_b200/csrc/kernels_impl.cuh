@@ -178,9 +178,9 @@ unsigned blocks_of(unsigned units, int tpb) {
 
 // Blocks of a launch over `units` pure units, and how they are laid out. Two units per warp where the blocks
 // still fill the device (148 SMs, 10 or more blocks each) several times over: a block's start costs about a tenth
-// of a one-unit block's life (D3Q19 FP32 160^3: 110.5 us with one, 106.6 with two, 113 with eight); smaller
-// lattices need the blocks to even out the end (97^3: 27.3 / 26.8 / 29.8; D2Q9 1024x512, 8192 blocks of one unit: BGK
-// 9.4 / 8.5, MRT 9.0 / 7.5). `four`: four units from 74,000 blocks, on D3Q19 and FP16C lattices (256^3 box, two / four:
+// of a one-unit block's life (D3Q19 FP32 160^3: 119 us with one, 112 with two, 115 with eight; D2Q9 1024x512 MRT,
+// 8192 blocks of one unit: 8.2 / 7.8 / 9.3); smaller lattices need the blocks to even out the end (97^3: 25.9 / 26.1 /
+// 31.0; 48^3: 5.6 / 7.2 / 16). `four`: four units from 74,000 blocks, on D3Q19 and FP16C lattices (256^3 box, two / four:
 // D3Q19 FP32 TRT 414 / 399, F16 MRT 417 / 412, D3Q27 FP16C MRT 733 / 721; D3Q27 F16 BGK 588 / 599 and FP32 BGK
 // 568 / 570, so not there).
 unsigned plan(unsigned units, int tpb, unsigned list_blocks, bool four, unsigned& run, unsigned& spread) {

@@ -19,9 +19,9 @@ namespace wk {
 // ---------------------------------------------------------------- cache policy of the population loads
 // Each population is read once per step and its line is dead after that, while the lines a step writes are the
 // next step's input. Where one state buffer fits the L2 (126 MB), reading it evict-first keeps the written
-// one there (D2Q9 FP32 2048x1024, 75 MB a buffer: 26.4 -> 23.8 us a step; D3Q19 97^3: 26.1 -> 23.6). Larger
+// one there (D2Q9 FP32 2048x1024, 75 MB a buffer: 24.0 -> 22.0 us a step; D3Q19 97^3: 28.0 -> 26.1). Larger
 // lattices read with the normal policy: neighbouring warps share the sectors at the ends of their unaligned loads,
-// which evict-first loses in between (D3Q19 256x128x128: 108.4 us, 114.8 evict-first).
+// which evict-first loses in between (D3Q19 256x128x128: 110.0 us, 115.6 evict-first).
 using L2Policy = unsigned long long;
 __device__ __forceinline__ L2Policy read_policy(bool evict_first) {
     L2Policy first, normal;

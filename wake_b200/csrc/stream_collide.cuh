@@ -138,18 +138,15 @@ __device__ __forceinline__ void gather_pure(const typename Codec<S>::T* __restri
     }
 }
 
-// Pull f^{k+1}(x) out of g^k. `bb` gets bit q when the pull of q bounced off a
-// solid or moving-wall node (in range), which marks the momentum-exchange link
-// (x, opp(q)).
+// Pull f^{k+1}(x) out of g^k.
 template <int Q, int S>
 __device__ __forceinline__ void gather(const typename Codec<S>::T* __restrict__ fin, const Geo& G,
                                        const uint8_t* __restrict__ flags, const Links& B, int x, int y, int z,
-                                       long long i, uint8_t fl, float f[Q], unsigned& bb) {
+                                       long long i, uint8_t fl, float f[Q]) {
     using L = Lat<Q>;
     using C = Codec<S>;
     const long long P = G.pitch;
     const int nx = G.nx, ny = G.ny, nz = G.nz;
-    bb = 0u;
     if (fl & FL_FAST) {
         gather_pure<Q, S>(fin, G, x, y, z, f);
         if (fl & FL_ZH_IN) zou_he_inlet<Q>(f, G.uin);
@@ -172,10 +169,8 @@ __device__ __forceinline__ void gather(const typename Codec<S>::T* __restrict__ 
         const uint8_t t = flags[s] & FL_TYPE;
         if (t == CT_SOLID) {
             f[q] = C::load(fin + o * P + i, L::w(o));
-            bb |= 1u << q;
         } else if (t == CT_MOVING_WALL) {
             f[q] = C::load(fin + o * P + i, L::w(o)) + G.mom[q];
-            bb |= 1u << q;
         } else {
             f[q] = C::load(fin + q * P + s, L::w(q));
         }
@@ -420,8 +415,7 @@ __global__ void __launch_bounds__(512) k_materialise(const void* fin_v, const ui
 #pragma unroll
         for (int q = 0; q < Q; ++q) f[q] = C::load(fin + q * geo.pitch + i, L::w(q));
     } else {
-        unsigned bb;
-        gather<Q, S>(fin, geo, flags, links, x, y, z, i, fl, f, bb);
+        gather<Q, S>(fin, geo, flags, links, x, y, z, i, fl, f);
     }
     if (out.f) {
 #pragma unroll

@@ -687,8 +687,11 @@ __global__ void __launch_bounds__(WK_FAST_MAX_THREADS, (cell_min_blocks<Q, COLL,
         }
         return;
     }
+    unsigned warp = threadIdx.x >> 5;
+    // known to the compiler as the warp's: its table entry is then addressed once for the warp (512 channels FP16 388 -> 375 us)
+    if constexpr (W == 1u) warp = __shfl_sync(0xffffffffu, warp, 0);
     walk(
-        block, threadIdx.x >> 5, b.npure * W, b.run, [&](unsigned u) { return __ldg(b.pure + u / W); },
+        block, warp, b.npure * W, b.run, [&](unsigned u) { return __ldg(b.pure + u / W); },
         [&](unsigned u, uint2 r) {
             const BatchDom& d = b.dom[r.x & 0xffffffu];
             const StepArgs& a = d.a;

@@ -10,8 +10,8 @@
 // resident per SM. Two nodes per thread: 64 x 8 gives D3Q19 / D3Q27 128 registers (16 warps per SM), which their 38 / 54
 // loads in flight need without spills. Sphere channel FP32 256x128x128, 160^3, 48^3: 110, 112, 5.6 us a step; at
 // 96 registers (20 warps) 117, 117, 5.9. D2Q9 carries half the values: 64 registers and 32 warps (2048x1024:
-// 22.0 us, 25.2 with 96 registers); 80 where a batch's arguments have to be read (60 channels: 53.6 us a step, 58.1
-// with 96 registers).
+// 22.0 us, 25.2 with 96 registers); 72 where a batch's arguments have to be read (512 channels FP32 / FP16, 32 threads: 413 /
+// 345 us a step, 431 / 375 with 80 registers, 418 / 342 with 64; 60 channels 50.9 / 39.7, 52.5 / 41.7, 51.8 / 41.3).
 // The FP32 D3Q27 MRT takes 168 with Smagorinsky's tau and in a batch: with 128 it spills 2.2 KB a thread (256^3 box with
 // Smagorinsky 664 us a step, 920 with 128; batch of two 160^3 boxes 345, 473).
 #ifndef WK_PAIRS27_MIN_BLOCKS
@@ -27,7 +27,7 @@
 #define WK_PAIRS9_MIN_BLOCKS 16
 #endif
 #ifndef WK_PAIRS9_BATCH_MIN_BLOCKS
-#define WK_PAIRS9_BATCH_MIN_BLOCKS 12
+#define WK_PAIRS9_BATCH_MIN_BLOCKS 14
 #endif
 
 namespace wk {

@@ -182,7 +182,7 @@ unsigned blocks_of(unsigned units, int tpb) {
 // 8192 blocks of one unit: 8.2 / 7.8 / 9.3); smaller lattices need the blocks to even out the end (97^3: 25.9 / 26.1 /
 // 31.0; 48^3: 5.6 / 7.2 / 16). `four`: four units from 74,000 blocks, on D3Q19 and FP16C lattices (256^3 box, two / four:
 // D3Q19 FP32 TRT 414 / 399, F16 MRT 417 / 412, D3Q27 FP16C MRT 733 / 721; D3Q27 F16 BGK 588 / 599 and FP32 BGK
-// 568 / 570, so not there).
+// 568 / 570, so not there), and in batches but D3Q27 ones (512 channels FP32 / FP16 431 / 375 and 404 / 348).
 unsigned plan(unsigned units, int tpb, unsigned list_blocks, bool four, unsigned& run, unsigned& spread) {
     unsigned blocks = blocks_of(units, tpb);
     run = blocks >= 148u * 500u && four ? 4u : (blocks >= 148u * 40u ? 2u : 1u);
@@ -216,7 +216,7 @@ void cells_one(StepArgs& a, int tpb, cudaStream_t st) {
 template <int C, int S, bool LES, bool TH>
 void batch_one(BatchArgs& b, int tpb, cudaStream_t st) {
     b.list_blocks = blocks_of(b.nlisted, tpb);
-    const unsigned blocks = plan(b.npure * pure_units<kQ, C, S, false>(), tpb, b.list_blocks, false, b.run, b.spread);
+    const unsigned blocks = plan(b.npure * pure_units<kQ, C, S, false>(), tpb, b.list_blocks, kQ != 27, b.run, b.spread);
     if (blocks) launch_step(k_step_cells_batch<kQ, C, S, LES, TH>, blocks, tpb, st, b, true);
 }
 template <int C, int S, bool LES>

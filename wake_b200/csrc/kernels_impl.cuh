@@ -180,12 +180,12 @@ unsigned blocks_of(unsigned units, int tpb) {
 // still fill the device (148 SMs, 10 or more blocks each) several times over: a block's start costs about a tenth
 // of a one-unit block's life (D3Q19 FP32 160^3: 119 us with one, 112 with two, 115 with eight; D2Q9 1024x512 MRT,
 // 8192 blocks of one unit: 8.2 / 7.8 / 9.3); smaller lattices need the blocks to even out the end (97^3: 25.9 / 26.1 /
-// 31.0; 48^3: 5.6 / 7.2 / 16). `four`: four units from 74,000 blocks, on D3Q19 and FP16C lattices (256^3 box, two / four:
+// 31.0; 48^3: 5.6 / 7.2 / 16). `four`: four units from 59,200 blocks, on D3Q19 and FP16C lattices (256^3 box, two / four:
 // D3Q19 FP32 TRT 414 / 399, F16 MRT 417 / 412, D3Q27 FP16C MRT 733 / 721; D3Q27 F16 BGK 588 / 599 and FP32 BGK
 // 568 / 570, so not there), and in batches but D3Q27 ones (512 channels FP32 / FP16 431 / 375 and 404 / 348).
 unsigned plan(unsigned units, int tpb, unsigned list_blocks, bool four, unsigned& run, unsigned& spread) {
     unsigned blocks = blocks_of(units, tpb);
-    run = blocks >= 148u * 500u && four ? 4u : (blocks >= 148u * 40u ? 2u : 1u);
+    run = blocks >= 148u * 400u && four ? 4u : (blocks >= 148u * 40u ? 2u : 1u);
     blocks = list_blocks + (blocks + run - 1u) / run;
     spread = 0;
     while (list_blocks && (static_cast<unsigned long long>(list_blocks) << (spread + 1)) <= blocks / 5ull * 3ull) ++spread;

@@ -417,7 +417,7 @@ def batched_leg(storage, n_domains=512, steps=STEPS_PER_SIM, warmup=20, baseline
         g.close()
     per_job_ms = ranks.max(per_job_ms)
     base_nodes = int(ranks.sum(base_nodes))
-    bpn = 2 * 9 * (4 if storage == "f32" else 2) + 1
+    bpn = 2 * 9 * (4 if storage == "f32" else 2)
     sims = n_domains * steps / STEPS_PER_SIM / (ms * 1e-3)
     base_sims = baseline_jobs * steps / STEPS_PER_SIM / (per_job_ms * 1e-3)
     return {"metric": "sims/s", "value": sims, "unit": "sims/s", "storage": storage, "domains": n_domains,
@@ -612,7 +612,7 @@ def tgv_leg(L=384, steps=5000, every=500, graph=20):
            "graph_steps": graph, "checkpoints": rows}
     peak, _ = hbm_peak()
     for st in grids:
-        bpn = 2 * 27 * (4 if st == "f32" else 2) + 1
+        bpn = 2 * 27 * (4 if st == "f32" else 2)
         sec = ms[st] * 1e-3
         mlups = n * timed_steps_done / sec / 1e6 if sec > 0 else None
         gbs = bpn * n * timed_steps_done / sec / 1e9 if sec > 0 else None
